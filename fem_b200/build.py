@@ -9,13 +9,18 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libfemh.so")
-SOURCES = [os.path.join(CSRC, "engine.cu"), os.path.join(HERE, "host", "femh_host.cpp")]
-HEADERS = [os.path.join(CSRC, f) for f in ("femh_common.cuh", "stencil.cuh", "kernels.cuh")] + [
+SOURCES = [os.path.join(CSRC, f) for f in (
+    "engine.cu", "stencil_f32_sweep.cu", "stencil_f32_apply.cu", "stencil_f64_sweep.cu", "stencil_f64_apply.cu")] + [
+    os.path.join(HERE, "host", "femh_host.cpp")]
+HEADERS = [os.path.join(CSRC, f) for f in (
+    "femh_common.cuh", "stencil.cuh", "stencil_launch.cuh", "kernels.cuh", "state.cuh")] + [
     os.path.join(HERE, "host", "femh_host.hpp")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
@@ -24,7 +29,6 @@ FLAGS = [
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-O3",
     "--expt-relaxed-constexpr",
-    "-shared",
     "-ccbin", "g++",
 ]
 
@@ -40,19 +44,27 @@ def _stale() -> bool:
 def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False) -> str:
     if not force and not _stale():
         return LIB
-    cmd = [NVCC, *FLAGS, "-o", LIB, *SOURCES, "-lcudart"]
-    if ptxas_v:
-        cmd.insert(1, "-Xptxas=-v")
-    if verbose:
-        print(" ".join(cmd), file=sys.stderr)
     env = dict(os.environ)
     env.pop("CC", None)
     env.pop("CXX", None)
-    res = subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True, env=env)
-    if res.returncode != 0:
-        raise RuntimeError(f"nvcc failed ({res.returncode}):\n{res.stdout}\n{res.stderr}")
-    if verbose or ptxas_v:
-        sys.stderr.write(res.stdout + res.stderr)
+    flags = [*FLAGS, "-Xptxas=-v"] if ptxas_v else FLAGS
+    # one nvcc per source, side by side (the stencil instantiations take minutes each), then the link
+    with tempfile.TemporaryDirectory() as tmp, ThreadPoolExecutor(len(SOURCES)) as pool:
+        objs = [os.path.join(tmp, os.path.basename(src) + ".o") for src in SOURCES]
+        cmds = [[NVCC, *flags, "-c", "-o", o, src] for o, src in zip(objs, SOURCES)]
+        link = [NVCC, *FLAGS, "-shared", "-o", LIB, *objs, "-lcudart"]
+
+        def run(cmd):
+            if verbose:
+                print(" ".join(cmd), file=sys.stderr)
+            res = subprocess.run(cmd, cwd=CSRC, capture_output=True, text=True, env=env)
+            if res.returncode != 0:
+                raise RuntimeError(f"nvcc failed ({res.returncode}):\n{res.stdout}\n{res.stderr}")
+            if verbose or ptxas_v:
+                sys.stderr.write(res.stdout + res.stderr)
+
+        list(pool.map(run, cmds))
+        run(link)
     return LIB
 
 

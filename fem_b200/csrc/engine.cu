@@ -5,43 +5,10 @@
 // (setParam -> topoOptLib Homogenize -> copyPeriodicU -> energy loop; df) and
 // SamplesGenerator/NumericalCoarseningUsingMultiGrid.cpp:221-345.  There is no
 // CPU fallback: every numeric step below is one of this library's kernels.
-#include <algorithm>
-#include <chrono>
-#include <cmath>
-#include <cstdio>
-#include <cstdint>
-#include <cstdlib>
-#include <cstring>
-#include <functional>
-#include <map>
-#include <memory>
-#include <mutex>
-#include <stdexcept>
-#include <string>
-#include <vector>
-
-#include "../../include/femh.h"
 #include "kernels.cuh"
-
-using namespace femh;
+#include "state.cuh"
 
 namespace {
-
-struct FemhError {
-  int code;
-  std::string msg;
-};
-
-#define CK(x)                                                                              \
-  do {                                                                                     \
-    cudaError_t e_ = (x);                                                                  \
-    if (e_ != cudaSuccess) {                                                               \
-      char b_[512];                                                                        \
-      snprintf(b_, sizeof b_, "%s failed: %s (%s:%d)", #x, cudaGetErrorString(e_), __FILE__, \
-               __LINE__);                                                                  \
-      throw FemhError{e_ == cudaErrorMemoryAllocation ? FEMH_E_OOM : FEMH_E_CUDA, b_};      \
-    }                                                                                      \
-  } while (0)
 
 // ------------------------------------------------------------ host math ---
 // Element matrix of a unit cube (h = 1) for the engineering-Voigt material
@@ -295,95 +262,6 @@ ElemConst host_elemconst(const double K[576]) {
   return ec;
 }
 
-// ------------------------------------------------------------- device mem ---
-struct Arena {
-  std::vector<void*> ptrs;
-  size_t held = 0;            // bytes allocated
-  size_t limit = SIZE_MAX;    // FEMH_ARENA_LIMIT_BYTES (tests only): fail like a full device beyond it
-  void* get(size_t bytes) {
-    if (bytes == 0) bytes = 16;
-    if (bytes > limit - held) throw FemhError{FEMH_E_OOM, "device memory limit of this handle reached"};
-    void* p = nullptr;
-    CK(cudaMalloc(&p, bytes));
-    ptrs.push_back(p);
-    held += bytes;
-    return p;
-  }
-  template <typename T> T* arr(size_t n) { return static_cast<T*>(get(n * sizeof(T))); }
-  void release() {
-    for (void* p : ptrs) cudaFree(p);
-    ptrs.clear();
-    held = 0;
-  }
-  ~Arena() { release(); }
-};
-
-template <typename T>
-T* upload(Arena& ar, const std::vector<T>& v, cudaStream_t s) {
-  T* d = ar.arr<T>(std::max<size_t>(v.size(), 1));
-  if (!v.empty()) CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
-  return d;
-}
-
-struct UnitList {
-  std::vector<StencilUnit> su;
-  StencilUnit* d_su = nullptr;
-  std::vector<NodeUnit> nu;
-  NodeUnit* d_nu = nullptr;
-  // persistent staged kernel (variant 7): CTA b runs units [cta[b], cta[b+1])
-  std::vector<int> cta;
-  int* d_cta = nullptr;
-  int cta_cap = 0;   // entries allocated at d_cta
-};
-
-// Stencil units of one z extent: entries [b, e) of a unit list sorted by z extent.
-struct UnitGroups {
-  std::vector<int> nz, b, e;
-};
-
-struct Level {
-  std::vector<CellDesc> cells;
-  CellDesc* d_cells = nullptr;
-  long long ntot = 0, nodes_smooth = 0;
-  int level = 0;
-  int NT = 256, maxnz = 1;
-  int nz_spec = 0;   // > 0: every cell of the level has this z extent (specialised kernel)
-  int chunk = 0;     // x-chunk length of the stencil units (0 = heuristic), set by the autotuner
-  int variant = 2;   // stencil kernel (femh_config::stencil_variant numbering)
-  bool bulk_ok = false;     // the bulk-copy staged FP32 kernel (variant 5) can run on this level
-  bool bulk_ok64 = false;   // the bulk-copy staged FP64 kernel (variant 6) can run on this level
-  // cells of several z extents, each one with a compile-time kernel (a batch
-  // of uneven cells): the unit lists are sorted by z extent and each extent
-  // launches its own specialised kernel
-  bool grouped = false;
-  UnitGroups gall, gsmooth, g64;
-  // level 0 of the mixed modes also runs FP64 operator applies (CG / true
-  // residual): they get their own tuned layout (FP64 kernels spill in the
-  // layout that suits FP32)
-  bool use64 = false;
-  int variant64 = 1, chunk64 = 0;
-  std::vector<StencilUnit> su64;
-  StencilUnit* d_su64 = nullptr;
-  std::vector<int> su64_sb, su64_se;
-  int *d_su64_sb = nullptr, *d_su64_se = nullptr;
-  UnitList all, smooth;      // all cells / cells that continue to a coarser level
-  std::vector<int> su_sb, su_se, nu_sb, nu_se;   // slot ranges per cell (all lists)
-  int *d_su_sb = nullptr, *d_su_se = nullptr, *d_nu_sb = nullptr, *d_nu_se = nullptr;
-  std::vector<int> coarse_list;                  // cells whose coarsest level this is
-  int* d_coarse_list = nullptr;
-  long long* d_aoff = nullptr;
-  double* d_A = nullptr;
-  double* d_Awork = nullptr;
-  int* d_cstat = nullptr;
-  int coarse_maxm = 0;
-  void* kc = nullptr;     // TC
-  float* invd = nullptr;
-  float* binv = nullptr;  // node-block Jacobi: [node][6] symmetric 3x3 inverses (block_jacobi)
-  void* xa = nullptr;     // level vectors (TV)
-  void* xb = nullptr;
-  void* bv = nullptr;
-};
-
 int pow2ceil(int v) {
   int p = 1;
   while (p < v) p <<= 1;
@@ -392,157 +270,7 @@ int pow2ceil(int v) {
 
 }  // namespace
 
-// ============================================================== handle ===
-struct femh_handle {
-  femh_config cfg{};
-  int device = 0;
-  cudaStream_t own_stream = nullptr, stream = nullptr;
-  std::string err;
-  long long launches = 0;
-  double K0[576];
-  HadK hk{};
-  HadK hk_force{};   // Hadamard factors of host_k0_force (femh_force_tensors)
-  ElemConst ec{};
-  ElemConst* d_ec = nullptr;
-  double* d_K0 = nullptr;
-  std::vector<double> w_pre, w_post;   // damping weight of each smoothing sweep
-  Arena perm;   // lives as long as the handle
-
-  // setup cache
-  std::vector<int> shape_key;
-  std::vector<double> h_key;
-  int prec_key = -1, solver_key = -1, bf16_key = -1;
-  Arena setup;
-  std::vector<Level> levels;
-  std::map<std::string, int> tune_cache;   // autotuned x-chunk per level signature
-  int ncells = 0;
-  std::vector<long long> cell_vox;   // voxels per cell
-  std::vector<long long> cell_off;   // fine offsets
-  long long nvox = 0;
-  // fine-level FP64 arrays
-  double* rho_in = nullptr;     // packed input rho
-  double* rho_used = nullptr;
-  double* kc64 = nullptr;
-  double* b64 = nullptr;        // [6][3][nvox]
-  double* x64 = nullptr;        // solution chi
-  double* r64 = nullptr;
-  void* cg_x = nullptr;         // inner CG vectors (TV / TP)
-  void* cg_r = nullptr;
-  void* cg_p = nullptr;
-  void* cg_q = nullptr;
-  void* cg_rm = nullptr;        // FP32 copy of the FP64 residual (level-0 rhs of an FP32 V-cycle)
-  CGState* d_state = nullptr;
-  BlockCG* d_bcg = nullptr;     // block PCG step matrices per cell
-  double* d_part_g = nullptr;   // block PCG 6x6 partials [2][sub-slots][36]
-  double* d_part_b = nullptr;   // block PCG ||r||^2 partials [sub-slots][6]
-  size_t part_g_slots = 0;      // slots of level 0 before any compaction (units keep their slot)
-  int bsub = 1;                 // block PCG update / direction: CTAs per level-0 node unit
-  int bsub_g = 1;               // block PCG Gram kernels: CTAs per level-0 node unit
-  std::vector<CGState> state;
-  double* d_part_s = nullptr;   // stencil partials [slots][6]
-  double* d_part_n = nullptr;   // node partials [slots][6][2]
-  double* d_part_z = nullptr;   // node partials [slots][6]
-  double* d_part_e = nullptr;   // energy partials [slots][21]
-  double* d_C = nullptr;        // [ncells][36]
-  double* d_W = nullptr;        // [ncells][21]
-  double* d_stage = nullptr;    // output staging (dCdrho, fields, apply), allocated on first use
-  size_t stage_n = 0;           // doubles in d_stage
-  // field chain rule: voxels of each field parameter (CSR), cached by the map's hash
-  int* d_fmap = nullptr;        // [nparam + 1] offsets, then [nmapped] voxel indices
-  size_t fmap_n = 0;            // ints allocated
-  unsigned long long fmap_key = 0;
-  int fmap_nparam = -1;
-  double* d_nrm = nullptr;      // [ncells][6]
-  bool solved = false;
-  bool have_x = false;   // x64 holds the last solution of these cells (warm starts)
-  std::vector<double> C_last;
-
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  int wait_limit = kWaitLimit;   // try_wait rounds of the staged kernels' stage waits
-  int nsm = 1;                   // multiprocessors of the device (persistent stencil CTAs)
-  // persistent stencil CTAs are split evenly over the six load cases; the inner
-  // solves of defect correction finish their load cases at different times
-  // (the CTAs of a finished one would idle), so they run one CTA per unit
-  bool persist_ok = true;
-  int* d_loop = nullptr;         // CG iterations run on the device in the current solve (WHILE-node count)
-  int* d_err = nullptr;   // [0] set by a stencil kernel whose bounded wait ran out,
-                          // [1] by k_coef on a NaN, infinite or negative density
-
-  // measurement: per-kernel-class CUDA-event timing (femh_profile), and the
-  // count of kernel executions including CUDA-graph replays
-  bool prof = false;
-  bool capturing = false;
-  long long cap_count = 0;
-  struct KStat {
-    long long launches = 0;
-    double ms = 0, bytes = 0;
-  };
-  std::map<std::string, KStat> kstats;
-  struct Pend {
-    std::string name;
-    cudaEvent_t a, b;
-    double bytes;
-  };
-  std::vector<Pend> pend;
-  std::vector<cudaEvent_t> evpool;
-};
-
 namespace {
-
-#define LAUNCH_CHECK(H)                          \
-  do {                                           \
-    CK(cudaGetLastError());                      \
-    if ((H)->capturing) (H)->cap_count++;        \
-    else (H)->launches++;                        \
-  } while (0)
-
-cudaEvent_t pool_event(femh_handle* H) {
-  if (!H->evpool.empty()) {
-    cudaEvent_t e = H->evpool.back();
-    H->evpool.pop_back();
-    return e;
-  }
-  cudaEvent_t e;
-  CK(cudaEventCreate(&e));
-  return e;
-}
-
-// Times the launches issued in its scope when profiling is on (graphs are
-// not captured then, so every launch is timed on the handle's stream).
-struct Prof {
-  femh_handle* H;
-  const char* name;
-  double bytes;
-  cudaEvent_t a = nullptr;
-  Prof(femh_handle* h, const char* n, double b) : H(h), name(n), bytes(b) {
-    if (H->prof && !H->capturing) {
-      a = pool_event(H);
-      CK(cudaEventRecord(a, H->stream));
-    }
-  }
-  ~Prof() {
-    if (a) {
-      cudaEvent_t b = pool_event(H);
-      if (cudaEventRecord(b, H->stream) == cudaSuccess) H->pend.push_back({name, a, b, bytes});
-    }
-  }
-};
-
-void prof_resolve(femh_handle* H) {
-  if (H->pend.empty()) return;
-  CK(cudaStreamSynchronize(H->stream));
-  for (auto& p : H->pend) {
-    float ms = 0;
-    CK(cudaEventElapsedTime(&ms, p.a, p.b));
-    auto& k = H->kstats[p.name];
-    k.launches++;
-    k.ms += ms;
-    k.bytes += p.bytes;
-    H->evpool.push_back(p.a);
-    H->evpool.push_back(p.b);
-  }
-  H->pend.clear();
-}
 
 void set_err(femh_handle* h, const std::string& m) {
   if (h) h->err = m;
@@ -595,18 +323,6 @@ void add_node_units(std::vector<NodeUnit>& out, int cellidx, long long nn, int& 
 }
 
 template <typename T> size_t esize() { return sizeof(T); }
-
-// Threads per CTA of a stencil variant on a level: the packed two-row kernel
-// needs up to ~160 registers a thread, so it runs 384-thread CTAs where its
-// tiles still hold at least two thread rows.
-int variant_nt(int level_nt, int maxnz, int variant) {
-  if ((variant == 4 || variant == 5 || variant == 7) && level_nt > 384 && 384 >= 2 * maxnz) return 384;
-  return level_nt;
-}
-
-// z extents with compile-time kernels, and their threads per CTA.
-bool spec_nz(int nz) { return nz == 16 || nz == 24 || nz == 32 || nz == 48 || nz == 64 || nz == 128 || nz == 256; }
-int spec_nt(int nz) { return (nz == 24 || nz == 48) ? 480 : 512; }
 
 // Threads per CTA that a cell's stencil units are cut for.
 int cell_nt(const Level& L, const CellDesc& cd, int variant) {
@@ -667,261 +383,7 @@ void build_cta_table(femh_handle* H, const Level& L, UnitList& ul, bool upload_n
 
 }  // namespace
 
-// ======================================================== kernel launch ===
 namespace {
-
-template <typename T, int NT, int OUT, int NZ, typename TIn, typename TOut, typename TB, typename TC>
-void stencil_go(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, TOut, TB, TC>& a, int variant) {
-  static bool attr1 = false, attr2 = false, attr3 = false;
-  if constexpr (std::is_same<T, float>::value) {
-    if (variant == 3) {   // two load cases per CTA in packed FP32x2 lanes
-      auto fn3 = stencilp_kernel<NT, OUT, NZ, TIn, TOut, TB, TC>;
-      if (!attr3) {
-        CK(cudaFuncSetAttribute(fn3, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        attr3 = true;
-      }
-      fn3<<<dim3(grid.x, kNumRhs / 2), NT, smem, H->stream>>>(a);
-      LAUNCH_CHECK(H);
-      return;
-    }
-  }
-  if (variant == 2) {
-    auto fn2 = stencil2_kernel<T, NT, OUT, NZ, TIn, TOut, TB, TC>;
-    if (!attr2) {
-      CK(cudaFuncSetAttribute(fn2, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr2 = true;
-    }
-    fn2<<<grid, NT, smem, H->stream>>>(a);
-    LAUNCH_CHECK(H);
-    return;
-  }
-  bool& attr = attr1;
-  auto fn = stencil_kernel<T, NT, OUT, NZ, TIn, TOut, TB, TC>;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
-  fn<<<grid, NT, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
-}
-
-// Two voxel rows per thread in packed FP32x2 lanes (variant 4).
-template <int NT, int OUT, int NZ, typename TIn, typename TOut, typename TB, typename TC>
-void stencil_go4(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, TOut, TB, TC>& a) {
-  static bool attr = false;
-  auto fn = stencil2p_kernel<NT, OUT, NZ, TIn, TOut, TB, TC>;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
-  fn<<<grid, NT, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
-}
-
-// Two voxel rows per thread in packed FP32x2 lanes, inputs staged by bulk copies (variant 5).
-template <int NT, int OUT, int NZ>
-void stencil_go5(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<float, float, float, float>& a) {
-  static bool attr = false;
-  auto fn = stencil2b_kernel<NT, OUT, NZ>;
-  if (!attr) {   // (a few bytes of static shared memory come on top)
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
-  fn<<<grid, NT, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
-}
-
-// FP64 operator, one voxel row per thread, inputs staged by bulk copies (variant 6).
-template <int NT, int OUT, int NZ, typename TIn>
-void stencil_go6(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, double, double, double>& a) {
-  static bool attr = false;
-  auto fn = stencil1b_kernel<NT, OUT, NZ, TIn>;
-  if (!attr) {   // (a few bytes of static shared memory come on top)
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    attr = true;
-  }
-  fn<<<grid, NT, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
-}
-
-// T = arithmetic type; in/out/b storage types as given.
-template <typename T, int OUT, typename TIn, typename TOut, typename TB, typename TC>
-void stencil(femh_handle* H, Level& L, bool smooth_only, const TIn* in, TOut* out, const TB* b,
-             const TC* kc, double* part, const CGState* stt, double omega) {
-  const bool use64 = sizeof(T) == 8 && L.use64 && !smooth_only;
-  UnitList& ul = smooth_only ? L.smooth : L.all;
-  const std::vector<StencilUnit>& units = use64 ? L.su64 : ul.su;
-  if (units.empty()) return;
-  int variant = use64 ? L.variant64 : L.variant;
-  if (!std::is_same<T, float>::value) {   // packed-FP32 kernels: FP64 twin with the same units
-    if (variant == 3) variant = 1;
-    if (variant == 4 || variant == 5 || variant == 7) variant = 2;
-  } else if (variant == 6) {   // the staged FP64 kernel's FP32 twin has the same units
-    variant = 1;
-  }
-  if (variant == 6) {   // bulk-copy staging: FP64 output / rhs / coefficients, aligned rows
-    const bool ok = std::is_same<TOut, double>::value && std::is_same<TB, double>::value &&
-                    std::is_same<TC, double>::value &&
-                    (std::is_same<TIn, double>::value || std::is_same<TIn, float>::value);
-    auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-    if (!(ok && L.bulk_ok64 && al(in) && al(out) && al(kc) && al(L.invd) && (!b || al(b)) && L.ntot % 4 == 0))
-      variant = 1;
-  }
-  bool persistent = false;
-  if (variant == 7) {   // the staged kernel as persistent CTAs over the list's CTA table
-    persistent = !use64 && !L.grouped && ul.cta.size() >= 2 && H->persist_ok;
-    variant = 5;
-  }
-  if (variant == 5) {   // bulk-copy staging: FP32 storage, 16-byte aligned rows, eligible level
-    const bool f32 = std::is_same<TIn, float>::value && std::is_same<TOut, float>::value &&
-                     std::is_same<TB, float>::value && std::is_same<TC, float>::value;
-    auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-    if (!(f32 && L.bulk_ok && al(in) && al(out) && al(kc) && al(L.invd) && (!b || al(b)) && L.ntot % 4 == 0)) {
-      variant = 4;
-      persistent = false;
-    }
-  }
-  StencilArgs<TIn, TOut, TB, TC> a;
-  a.cells = L.d_cells;
-  a.units = use64 ? L.d_su64 : ul.d_su;
-  a.u = in;
-  a.out = out;
-  a.b = b;
-  a.kc = kc;
-  a.invd = L.invd;
-  a.partials = part;
-  a.stt = stt;
-  a.ntot = L.ntot;
-  a.k = H->hk;
-  a.omega = omega;
-  a.err = H->d_err;
-  a.wait_limit = H->wait_limit;
-  a.cta_units = persistent ? ul.d_cta : nullptr;
-  a.binv = (OUT == OUT_JACOBI || OUT == OUT_JACOBI_DOT) ? L.binv : nullptr;
-  {
-    const HadK& k = H->hk;
-    const double kv[8] = {k.A, k.Bd - k.Bo, k.Bo, k.D1 - k.O1, k.O1, k.D2 - k.O2, k.O2, k.G};
-    for (int i = 0; i < 8; ++i) a.kp[i] = make_float2((float)kv[i], (float)kv[i]);
-  }
-  dim3 grid((unsigned)(persistent ? ul.cta.size() - 1 : units.size()), kNumRhs);
-  static const char* mode_names[] = {"apply", "apply_dot", "jacobi", "jacobi_dot", "resid"};
-  char nm[64];
-  snprintf(nm, sizeof nm, "stencil_%s_%s_L%d", sizeof(T) == 8 ? "f64" : "f32", mode_names[OUT], L.level);
-  // algorithmic bytes: only (cell, load case) pairs still iterating move data
-  double nodes = 0.0;
-  if (H->prof) {
-    for (const auto& cd : L.cells) {
-      if (smooth_only && cd.child < 0) continue;
-      int act = kNumRhs;
-      if (stt) {
-        act = 0;
-        for (int q = 0; q < kNumRhs; ++q) act += H->state[cd.id * kNumRhs + q].active ? 1 : 0;
-      }
-      nodes += (double)cd.nx * cd.ny * cd.nz * act / kNumRhs;
-    }
-  }
-  double per = 18.0 * (sizeof(TIn) + sizeof(TOut)) + sizeof(TC);
-  if (OUT >= OUT_JACOBI) per += 18.0 * sizeof(TB) + (OUT == OUT_RESID ? 0.0 : (L.binv ? 24.0 : 4.0));
-  std::string key(nm);
-  Prof prof_(H, H->prof ? H->kstats.emplace(key, femh_handle::KStat{}).first->first.c_str() : nm, nodes * per);
-  // launch on units of one z extent (nz_spec > 0: compile-time kernels) or on
-  // the level's runtime-z kernels (nz_spec = 0), lnt threads per CTA
-  auto launch = [&](int nz_spec, int lnt, int maxnz, dim3 grid, const StencilArgs<TIn, TOut, TB, TC>& a) {
-    const size_t smem =
-        variant == 3 ? sizeof(float4) * 12 * (size_t)lnt + 2 * sizeof(float2) * (size_t)(12 * lnt + 3 * maxnz) +
-                             64 * sizeof(double)
-        : variant == 2 ? sizeof(T) * (size_t)(2 * (6 * lnt + 3 * maxnz) + 24 * lnt) + 16 + 64 * sizeof(double)
-                       : 2 * sizeof(T) * (size_t)(15 * lnt + 3 * maxnz) + 16 + 64 * sizeof(double);
-    if constexpr (std::is_same<T, double>::value && std::is_same<TOut, double>::value &&
-                  std::is_same<TB, double>::value && std::is_same<TC, double>::value &&
-                  (std::is_same<TIn, double>::value || std::is_same<TIn, float>::value)) {
-      if (variant == 6) {
-        const size_t sm6 = stencil1b_smem_bytes(lnt, nz_spec, (int)sizeof(TIn));
-        switch (nz_spec) {
-          case 16: stencil_go6<512, OUT, 16>(H, grid, sm6, a); return;
-          case 24: stencil_go6<480, OUT, 24>(H, grid, sm6, a); return;
-          case 32: stencil_go6<512, OUT, 32>(H, grid, sm6, a); return;
-          case 48: stencil_go6<480, OUT, 48>(H, grid, sm6, a); return;
-          case 64: stencil_go6<512, OUT, 64>(H, grid, sm6, a); return;
-          case 128: stencil_go6<512, OUT, 128>(H, grid, sm6, a); return;
-          case 256: stencil_go6<512, OUT, 256>(H, grid, sm6, a); return;
-          default: throw FemhError{FEMH_E_ARG, "staged FP64 stencil on an ineligible level"};
-        }
-      }
-    }
-    if constexpr (std::is_same<TIn, float>::value && std::is_same<TOut, float>::value &&
-                  std::is_same<TB, float>::value && std::is_same<TC, float>::value) {
-      if (variant == 5) {   // eligible levels have a compile-time z extent and 384-thread tiles
-        const int nt = variant_nt(lnt, maxnz, 5);
-        const size_t sm5 = stencil2b_smem_bytes(nt, nz_spec);
-        switch (nz_spec) {
-          case 16: stencil_go5<384, OUT, 16>(H, grid, sm5, a); return;
-          case 24: stencil_go5<384, OUT, 24>(H, grid, sm5, a); return;
-          case 32: stencil_go5<384, OUT, 32>(H, grid, sm5, a); return;
-          case 48: stencil_go5<384, OUT, 48>(H, grid, sm5, a); return;
-          case 64: stencil_go5<384, OUT, 64>(H, grid, sm5, a); return;
-          case 128: stencil_go5<384, OUT, 128>(H, grid, sm5, a); return;
-          default: throw FemhError{FEMH_E_ARG, "bulk-copy stencil on an ineligible level"};
-        }
-      }
-    }
-    if constexpr (std::is_same<T, float>::value) {
-      if (variant == 4) {
-        const int nt = variant_nt(lnt, maxnz, 4);
-        const size_t sm4 =
-            sizeof(float2) * 18 * (size_t)nt + sizeof(float) * (6 * (size_t)maxnz + 2) + 64 * sizeof(double);
-        if (nt == 384) {
-          switch (nz_spec) {
-            case 16: stencil_go4<384, OUT, 16>(H, grid, sm4, a); return;
-            case 24: stencil_go4<384, OUT, 24>(H, grid, sm4, a); return;
-            case 32: stencil_go4<384, OUT, 32>(H, grid, sm4, a); return;
-            case 48: stencil_go4<384, OUT, 48>(H, grid, sm4, a); return;
-            case 64: stencil_go4<384, OUT, 64>(H, grid, sm4, a); return;
-            case 128: stencil_go4<384, OUT, 128>(H, grid, sm4, a); return;
-            default: stencil_go4<384, OUT, 0>(H, grid, sm4, a); return;
-          }
-        }
-        if (nz_spec == 256) {
-          stencil_go4<512, OUT, 256>(H, grid, sm4, a);
-          return;
-        }
-        switch (nt) {
-          case 128: stencil_go4<128, OUT, 0>(H, grid, sm4, a); return;
-          case 256: stencil_go4<256, OUT, 0>(H, grid, sm4, a); return;
-          case 512: stencil_go4<512, OUT, 0>(H, grid, sm4, a); return;
-          default: throw FemhError{FEMH_E_ARG, "unsupported stencil block size"};
-        }
-      }
-    }
-    switch (nz_spec) {   // compile-time z extent (threads fixed per extent)
-      case 16: stencil_go<T, 512, OUT, 16>(H, grid, smem, a, variant); return;
-      case 24: stencil_go<T, 480, OUT, 24>(H, grid, smem, a, variant); return;
-      case 32: stencil_go<T, 512, OUT, 32>(H, grid, smem, a, variant); return;
-      case 48: stencil_go<T, 480, OUT, 48>(H, grid, smem, a, variant); return;
-      case 64: stencil_go<T, 512, OUT, 64>(H, grid, smem, a, variant); return;
-      case 128: stencil_go<T, 512, OUT, 128>(H, grid, smem, a, variant); return;
-      case 256: stencil_go<T, 512, OUT, 256>(H, grid, smem, a, variant); return;
-      default: break;
-    }
-    switch (lnt) {
-      case 128: stencil_go<T, 128, OUT, 0>(H, grid, smem, a, variant); break;
-      case 256: stencil_go<T, 256, OUT, 0>(H, grid, smem, a, variant); break;
-      case 512: stencil_go<T, 512, OUT, 0>(H, grid, smem, a, variant); break;
-      default: throw FemhError{FEMH_E_ARG, "unsupported stencil block size"};
-    }
-  };
-  if (!L.grouped) {
-    launch(L.nz_spec, L.NT, L.maxnz, grid, a);
-    return;
-  }
-  // cells of several compile-time z extents: one launch per extent
-  const UnitGroups& gr = use64 ? L.g64 : (smooth_only ? L.gsmooth : L.gall);
-  for (size_t gi = 0; gi < gr.nz.size(); ++gi) {
-    StencilArgs<TIn, TOut, TB, TC> ag = a;
-    ag.units = a.units + gr.b[gi];
-    launch(gr.nz[gi], spec_nt(gr.nz[gi]), gr.nz[gi], dim3((unsigned)(gr.e[gi] - gr.b[gi]), kNumRhs), ag);
-  }
-}
 
 #define NODE_GRID(ul) dim3((unsigned)(ul).nu.size(), kNumRhs)
 
@@ -1660,6 +1122,14 @@ TM* vcycle(femh_handle* H, const TR* r0, double* dot_part) {
   return sol[0];
 }
 
+// V-cycle on the CG residual: the residual itself, or its copy rm in the
+// V-cycle's type where that differs.
+template <typename TM, typename TMC, typename TV>
+TM* vcycle_of(femh_handle* H, const TV* r, const TM* rm, double* dot_part) {
+  if constexpr (std::is_same<TM, TV>::value) return vcycle<TM, TMC, TM>(H, r, dot_part);
+  else return vcycle<TM, TMC, TM>(H, rm, dot_part);
+}
+
 // Solver precisions: TV = CG vectors, TP = search direction storage, TK = CG
 // operator coefficients, TM / TMC = multigrid level vectors / coefficients.
 template <typename TV, typename TP, typename TK, typename TM, typename TMC>
@@ -1724,7 +1194,7 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
                                                    H->w_pre[0], H->d_bcg, H->d_part_b, L0.ntot, L0.binv, nsub);
     LAUNCH_CHECK(H);
   }
-  TM* z = rm ? vcycle<TM, TMC, TM>(H, rm, nullptr) : vcycle<TM, TMC, TV>(H, r, nullptr);
+  TM* z = vcycle_of<TM, TMC>(H, r, rm, nullptr);
   block_gram<false, TM, TV>(H, "k_bgram_zr", (const TM*)z, (const TV*)r, part_a);
   block_gram<false, TV, TM>(H, "k_bgram_qz", (const TV*)q, (const TM*)z, part_b);
   {
@@ -1780,7 +1250,7 @@ void pcg_iteration(femh_handle* H, const typename PR::K* kcg, bool blk) {
   const bool fuse = fuse_rz(H);
   if (gmg) {
     double* dp = fuse ? H->d_part_z : nullptr;
-    z = rm ? vcycle<TM, TMC, TM>(H, rm, dp) : vcycle<TM, TMC, TV>(H, r, dp);
+    z = vcycle_of<TM, TMC>(H, r, rm, dp);
     if (!fuse) {
       Prof prof_(H, "k_dot", 0.0);
       k_dot<TM, TV><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, z, r, stt, H->d_part_z, L0.ntot);
@@ -1857,7 +1327,7 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
         k_binit<<<cdiv(nc, 128), 128, 0, s>>>(H->d_bcg, stt, nc);
         LAUNCH_CHECK(H);
       }
-      TM* z = rm ? vcycle<TM, TMC, TM>(H, rm, nullptr) : vcycle<TM, TMC, TV>(H, r, nullptr);
+      TM* z = vcycle_of<TM, TMC>(H, r, rm, nullptr);
       block_gram<false, TM, TV>(H, "k_bgram_zr", (const TM*)z, (const TV*)r, H->d_part_g);
       {
         Prof prof_(H, "k_bfin_rz", 0.0);
@@ -1875,7 +1345,7 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
   if (gmg && !blk) {
     const bool fuse = fuse_rz(H);
     double* dp = fuse ? H->d_part_z : nullptr;
-    TM* z = rm ? vcycle<TM, TMC, TM>(H, rm, dp) : vcycle<TM, TMC, TV>(H, r, dp);
+    TM* z = vcycle_of<TM, TMC>(H, r, rm, dp);
     if (!fuse) {
       Prof prof_(H, "k_dot", 0.0);
       k_dot<TM, TV><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, z, r, stt, H->d_part_z, L0.ntot);

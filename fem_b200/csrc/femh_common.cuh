@@ -59,6 +59,12 @@ struct HadK {
   double diag; // K0 diagonal entry (all 24 equal for the cube)
 };
 
+// Constants of the load and energy kernels, for h = 1 (scaled by h inside).
+struct ElemConst {
+  double g1[kNumRhs][24];      // K0(E=1,h=1) ue0^I(h=1), DOF 3a+c
+  double uhat0[kNumRhs][3][8]; // Hadamard transform of ue0^I(h=1)
+};
+
 // Per (cell, load case) CG state, kept on the device so that iterations can be
 // captured in a CUDA graph without host round trips.
 struct CGState {

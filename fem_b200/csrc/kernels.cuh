@@ -35,12 +35,6 @@ __host__ __device__ inline double law_dcoef(const MatLaw& m, double rho) {
   return 0.0;
 }
 
-// Constants of the load and energy kernels, for h = 1 (scaled by h inside).
-struct ElemConst {
-  double g1[kNumRhs][24];      // K0(E=1,h=1) ue0^I(h=1), DOF 3a+c
-  double uhat0[kNumRhs][3][8]; // Hadamard transform of ue0^I(h=1)
-};
-
 // (i, j, k) of node n of a cell; n < nx*ny*nz < 2^32, so 32-bit unsigned
 // division (far cheaper than 64-bit) is exact.
 __device__ __forceinline__ void node_ijk(long long n, int ny, int nz, int& i, int& j, int& k) {
