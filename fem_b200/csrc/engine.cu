@@ -234,9 +234,23 @@ std::vector<double> smooth_weights(int m, double lmax, double ratio, double omeg
   return w;
 }
 
-ElemConst host_elemconst(const double K[576]) {
+// Load and strain constants of the six unit macro strains.  The load is K0 ue0
+// in closed form: a uniform stress sigma = D eps puts (1/4) sum_d sigma_cd s_d(a)
+// on component c of corner a (s_d = +-1, unit cube), so opposite corners carry
+// equal and opposite values to the last bit and load cases that are alike on a
+// cell (a laminate's in-plane strains) get the same load bit for bit.
+ElemConst host_elemconst(double nu) {
   ElemConst ec{};
+  double D[6][6];
+  iso_voigt(nu, D);
   for (int I = 0; I < kNumRhs; ++I) {
+    const double sig[3][3] = {{D[0][I], D[5][I], D[4][I]}, {D[5][I], D[1][I], D[3][I]}, {D[4][I], D[3][I], D[2][I]}};
+    for (int a = 0; a < 8; ++a)
+      for (int c = 0; c < 3; ++c) {
+        double f = 0.0;
+        for (int d = 0; d < 3; ++d) f += 0.25 * sig[c][d] * ((a >> (2 - d)) & 1 ? 1.0 : -1.0);
+        ec.g1[I][3 * a + c] = f;
+      }
     double eps[3][3] = {};
     if (I < 3) eps[I][I] = 1;
     if (I == 3) eps[1][2] = eps[2][1] = 0.5;
@@ -246,11 +260,6 @@ ElemConst host_elemconst(const double K[576]) {
     for (int a = 0; a < 8; ++a) {
       const double x[3] = {double((a >> 2) & 1), double((a >> 1) & 1), double(a & 1)};
       for (int c = 0; c < 3; ++c) ue[3 * a + c] = eps[c][0] * x[0] + eps[c][1] * x[1] + eps[c][2] * x[2];
-    }
-    for (int p = 0; p < 24; ++p) {
-      double s = 0;
-      for (int q = 0; q < 24; ++q) s += K[p * 24 + q] * ue[q];
-      ec.g1[I][p] = s;
     }
     for (int c = 0; c < 3; ++c)
       for (int k = 0; k < 8; ++k) {
@@ -681,6 +690,7 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
   H->d_C = ar.arr<double>(nc * 36);
   H->d_W = ar.arr<double>(nc * 21);
   H->d_nrm = ar.arr<double>(nc * kNumRhs);
+  H->d_mean = ar.arr<double>(nc * kNumRhs * 3);
   H->shape_key = shapes;
   H->h_key = hs;
   H->prec_key = c.precision;
@@ -941,6 +951,8 @@ void autotune_levels(femh_handle* H, bool mg) {
   }
 }
 
+unsigned fin_blocks(int nc) { return cdiv((long long)nc * kNumRhs * 32, 128); }   // a warp per (cell, rhs)
+
 // coefficients on all levels + inverse diagonals + coarse factorisations
 template <typename TC>
 void prepare_operator(femh_handle* H) {
@@ -1009,13 +1021,25 @@ void prepare_operator(femh_handle* H) {
   // loads
   {
     Prof prof_(H, "k_rhs", 0.0);
-    k_rhs<double><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, H->kc64, H->d_ec, H->b64, L0.ntot);
+    k_rhs<true><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, H->kc64, H->d_ec, nullptr, L0.ntot,
+                                                  H->d_part_e, nullptr);
+    LAUNCH_CHECK(H);
+  }
+  {
+    Prof prof_(H, "k_rhs_mean", 0.0);
+    k_rhs_mean<<<fin_blocks(H->ncells), 128, 0, s>>>(L0.d_cells, L0.d_nu_sb, L0.d_nu_se, H->d_part_e, H->d_mean,
+                                                     H->ncells);
+    LAUNCH_CHECK(H);
+  }
+  {
+    Prof prof_(H, "k_rhs", 0.0);
+    k_rhs<false><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, H->kc64, H->d_ec, H->b64, L0.ntot,
+                                                   nullptr, H->d_mean);
     LAUNCH_CHECK(H);
   }
 }
 
 
-unsigned fin_blocks(int nc) { return cdiv((long long)nc * kNumRhs * 32, 128); }   // a warp per (cell, rhs)
 
 // The z . r product of the multigrid preconditioner comes out of the last
 // level-0 post-smoothing sweep when every level-0 cell is smoothed there (no
@@ -1848,7 +1872,7 @@ femh_status femh_create(femh_handle** out, const femh_config* cfg) {
       host_k0_force(cfg->nu, Kf);
       H->hk_force = host_hadk(Kf);
     }
-    H->ec = host_elemconst(H->K0);
+    H->ec = host_elemconst(cfg->nu);
     {
       const double lmax = host_jacobi_bound(H->K0, cfg->block_jacobi != 0);
       H->w_pre = smooth_weights(std::max(cfg->pre_smooth, 1), lmax, cfg->cheb_ratio, cfg->omega);
@@ -2161,7 +2185,7 @@ femh_status femh_fluctuation(femh_handle* H, double* chi_out, int out_on_device)
     double* tmp = stage(H, 18 * (size_t)nn);
     {
       Prof prof_(H, "k_layout", 0.0);
-      k_layout<true><<<cdiv(18 * nn, 256), 256, 0, H->stream>>>(H->x64, tmp, 0, nn, H->levels[0].ntot);
+      k_layout<true><<<cdiv(18 * nn, 256), 256, 0, H->stream>>>(H->x64, tmp, 0, nn, H->levels[0].ntot, 1);
       LAUNCH_CHECK(H);
     }
     to_host_or_dev(H, chi_out, tmp, 18 * nn, out_on_device);
@@ -2201,7 +2225,7 @@ femh_status femh_apply_operator(femh_handle* H, int nx, int ny, int nz, double h
     CK(cudaMemcpyAsync(tmp, u, sizeof(double) * 18 * nn, k_in, s));
     {
       Prof prof_(H, "k_layout", 0.0);
-      k_layout<false><<<cdiv(18 * nn, 256), 256, 0, s>>>(tmp, H->x64, 0, nn, L0.ntot);
+      k_layout<false><<<cdiv(18 * nn, 256), 256, 0, s>>>(tmp, H->x64, 0, nn, L0.ntot, 0);
       LAUNCH_CHECK(H);
     }
     if (f32) {
@@ -2222,7 +2246,7 @@ femh_status femh_apply_operator(femh_handle* H, int nx, int ny, int nz, double h
     }
     {
       Prof prof_(H, "k_layout", 0.0);
-      k_layout<true><<<cdiv(18 * nn, 256), 256, 0, s>>>(H->b64, tmp, 0, nn, L0.ntot);
+      k_layout<true><<<cdiv(18 * nn, 256), 256, 0, s>>>(H->b64, tmp, 0, nn, L0.ntot, 0);
       LAUNCH_CHECK(H);
     }
     to_host_or_dev(H, y, tmp, 18 * nn, on_device);
@@ -2414,7 +2438,7 @@ extern "C" femh_status femh_energy_noalloc(const femh_config* cfg, int nx, int n
   } catch (const FemhError&) {
     return FEMH_E_ARG;
   }
-  const ElemConst ec = host_elemconst(K);
+  const ElemConst ec = host_elemconst(cfg->nu);
   MatLaw law = make_law(*cfg);
   law.rho_bf16 = 0;
   const long long per = (nv + kNoAllocSlots - 1) / kNoAllocSlots;

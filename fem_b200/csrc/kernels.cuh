@@ -118,7 +118,7 @@ __global__ void k_invdiag(const CellDesc* cells, const NodeUnit* units, const TC
     for (int a = 0; a < 8; ++a)
       s += (double)kc[cd.off + lin(wrap(i - ((a >> 2) & 1), cd.nx), wrap(j - ((a >> 1) & 1), cd.ny),
                                    wrap(k - (a & 1), cd.nz), cd.ny, cd.nz)];
-    invd[cd.off + n] = (n == 0) ? 0.f : (float)(1.0 / (diag * s));
+    invd[cd.off + n] = (float)(1.0 / (diag * s));
   }
 }
 
@@ -128,7 +128,7 @@ __global__ void k_invdiag(const CellDesc* cells, const NodeUnit* units, const TC
 // diagonal, sigma_c = 1 - 2 bit_c(a) (d = K0 diagonal, o = K0[0][1]), so
 // D_n = d (sum kc) I + o T_n with T_n(c1, c2) = sum_e kc_e sigma_c1 sigma_c2.
 // binv[6 (cd.off + n) + k] = the symmetric inverse, k = xx, yy, zz, xy, xz, yz
-// (FP32; 0 at the pinned node 0).
+// (FP32).
 template <typename TC>
 __global__ void k_invblock(const CellDesc* cells, const NodeUnit* units, const TC* kc, double d, double o,
                            float* binv) {
@@ -154,7 +154,7 @@ __global__ void k_invblock(const CellDesc* cells, const NodeUnit* units, const T
     const double c00 = A * A - Z * Z, c11 = A * A - Y * Y, c22 = A * A - X * X;
     const double c01 = Y * Z - X * A, c02 = X * Z - Y * A, c12 = X * Y - A * Z;
     const double det = A * c00 + X * c01 + Y * c02;
-    const double r = (n == 0) ? 0.0 : 1.0 / det;
+    const double r = 1.0 / det;
     float* out = binv + 6 * (cd.off + n);
     out[0] = (float)(c00 * r);
     out[1] = (float)(c11 * r);
@@ -166,29 +166,50 @@ __global__ void k_invblock(const CellDesc* cells, const NodeUnit* units, const T
 }
 
 // Strain-driven load b^I_n = -sum_{e at n} c_e (K0(h) ue0^I(h))[a_n(e)]
-//   = -h * sum_e kc_e g1^I[a_n(e)]  (K0(h) = h K0(1), ue0(h) = h ue0(1), kc = c h).
-// Pinned node 0 gets 0.  One CTA per (unit, load case).
-template <typename TB>
-__global__ void k_rhs(const CellDesc* cells, const NodeUnit* units, const double* kc64,
-                      const ElemConst* ec, TB* b, long long ntot) {
+//   = -h * sum_e kc_e g1^I[a_n(e)]  (K0(h) = h K0(1), ue0(h) = h ue0(1), kc = c h),
+// without its net force.  The exact load has none, and the solver leaves the
+// three translations free, so it needs a load without one; and where the exact
+// load is zero (a uniform neighbourhood), rounding must not make one up: a
+// node's sum below its rounding bound, 8 u sum |kc_e g1|, is 0.  Two passes over the densities (8 B per node
+// each, against 144 B of load): SUM adds the load up, [slot][6][3] partials;
+// the other writes it less its mean per (cell, load case, component).
+// One CTA per (unit, load case).
+template <bool SUM>
+__global__ void k_rhs(const CellDesc* cells, const NodeUnit* units, const double* kc64, const ElemConst* ec,
+                      double* __restrict__ b, long long ntot, double* __restrict__ part,
+                      const double* __restrict__ mean) {
   const NodeUnit u = units[blockIdx.x];
   const int I = blockIdx.y;
   const CellDesc cd = cells[u.cell];
+  double v[3] = {0.0, 0.0, 0.0};
   #pragma unroll 4
   for (long long n = u.begin + threadIdx.x; n < u.end; n += blockDim.x) {
     int i, j, k;
     node_ijk(n, cd.ny, cd.nz, i, j, k);
-    double acc[3] = {0, 0, 0};
+    double acc[3] = {0, 0, 0}, size[3] = {0, 0, 0};
 #pragma unroll
     for (int a = 0; a < 8; ++a) {
       const double ke = kc64[cd.off + lin(wrap(i - ((a >> 2) & 1), cd.nx), wrap(j - ((a >> 1) & 1), cd.ny),
                                           wrap(k - (a & 1), cd.nz), cd.ny, cd.nz)];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) acc[c] += ke * ec->g1[I][3 * a + c];
+      for (int c = 0; c < 3; ++c) {
+        acc[c] += ke * ec->g1[I][3 * a + c];
+        size[c] += ke * fabs(ec->g1[I][3 * a + c]);
+      }
     }
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      st_val(b + ((long long)I * 3 + c) * ntot + cd.off + n, (n == 0) ? 0.0 : -cd.h * acc[c]);
+    for (int c = 0; c < 3; ++c) {
+      const double f = fabs(acc[c]) <= 8.0 * 1.1102230246251565e-16 * size[c] ? 0.0 : -cd.h * acc[c];
+      if (SUM) v[c] += f;
+      else b[((long long)I * 3 + c) * ntot + cd.off + n] = f - mean[(cd.id * kNumRhs + I) * 3 + c];
+    }
+  }
+  if (SUM) {
+    __shared__ double red[32 * 3];
+    block_reduce<3>(v, red);
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) part[((long long)u.slot * kNumRhs + I) * 3 + c] = v[c];
   }
 }
 
@@ -214,7 +235,7 @@ __global__ void k_cg_init(const CellDesc* cells, const NodeUnit* units, const TB
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const long long o = ((long long)rhs * 3 + c) * ntot + g;
-        const double rv = (n == 0) ? 0.0 : S.scale * (double)ld_val(b + o);
+        const double rv = S.scale * (double)ld_val(b + o);
         if (!keep_x) st_val(x + o, 0.0);
         st_val(r + o, rv);
         v[0] += rv * rv;
@@ -232,7 +253,7 @@ __global__ void k_cg_init(const CellDesc* cells, const NodeUnit* units, const TB
   }
 }
 
-// x += alpha p ; r -= alpha q (r = 0 at node 0) ; partial ||r||^2 and, for
+// x += alpha p ; r -= alpha q ; partial ||r||^2 and, for
 // Jacobi, r.(invd r).  For the multigrid preconditioner (z0 != nullptr) it
 // also writes the first damped-Jacobi sweep from zero: z0 = omega invd r, and,
 // when rm != nullptr, r in the V-cycle's storage type (the level-0 right-hand
@@ -259,7 +280,7 @@ __global__ void k_cg_update(const CellDesc* cells, const NodeUnit* units, TV* __
         const long long o = ((long long)rhs * 3 + c) * ntot + g;
         const double pv = (double)ld_val(p + o);
         const double xv = (double)ld_val(x + o) + al * pv;
-        const double rv = (n == 0) ? 0.0 : (double)ld_val(r + o) - al * (double)ld_val(q + o);
+        const double rv = (double)ld_val(r + o) - al * (double)ld_val(q + o);
         st_val(x + o, xv);
         st_val(r + o, rv);
         v[0] += rv * rv;
@@ -656,7 +677,7 @@ k_bupdate(const CellDesc* cells, const NodeUnit* units, TV* __restrict__ x, TV* 
             dr += al[i * 6 + j] * qv[i];
           }
           const long long o = ((long long)j * 3 + c) * ntot + g;
-          const double rj = (n == 0) ? 0.0 : (double)ld_val(r + o) - dr;
+          const double rj = (double)ld_val(r + o) - dr;
           st_val(x + o, (double)ld_val(x + o) + dx);
           st_val(r + o, rj);
           if (rm) st_val(rm + o, rj);
@@ -839,7 +860,8 @@ __global__ void k_fin_beta(CGState* stt, const int* slot_begin, const int* slot_
 
 // ---------------------------------------------------------- multigrid ---
 // Full-weighting restriction (transpose of trilinear prolongation):
-// bc(I) = sum_{d in {-1,0,1}^3} prod_s (1 - |d_s|/2) rf(2I + d); 0 at node 0.
+// bc(I) = sum_{d in {-1,0,1}^3} prod_s (1 - |d_s|/2) rf(2I + d).  The weights of a
+// fine node add up to 1, so a residual without net force stays one.
 // xc != nullptr: also the coarse level's first damped-Jacobi sweep from a zero
 // guess, xc = omega * invdc * bc (as stored), on the coarse cells that are
 // smoothed there (child >= 0; the others are solved directly).
@@ -858,21 +880,19 @@ __global__ void k_restrict(const CellDesc* fine, const CellDesc* coarse, const N
     int i, j, k;
     node_ijk(n, cc.ny, cc.nz, i, j, k);
     double acc[3] = {0, 0, 0};
-    if (n != 0) {
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int fi = wrap(2 * i + dx, cf.nx);
-        const double wx = dx ? 0.5 : 1.0;
-        for (int dy = -1; dy <= 1; ++dy) {
-          const int fj = wrap(2 * j + dy, cf.ny);
-          const double wy = wx * (dy ? 0.5 : 1.0);
+    for (int dx = -1; dx <= 1; ++dx) {
+      const int fi = wrap(2 * i + dx, cf.nx);
+      const double wx = dx ? 0.5 : 1.0;
+      for (int dy = -1; dy <= 1; ++dy) {
+        const int fj = wrap(2 * j + dy, cf.ny);
+        const double wy = wx * (dy ? 0.5 : 1.0);
 #pragma unroll
-          for (int dz = -1; dz <= 1; ++dz) {
-            const int fk = wrap(2 * k + dz, cf.nz);
-            const double w = wy * (dz ? 0.5 : 1.0);
-            const long long g = cf.off + lin(fi, fj, fk, cf.ny, cf.nz);
+        for (int dz = -1; dz <= 1; ++dz) {
+          const int fk = wrap(2 * k + dz, cf.nz);
+          const double w = wy * (dz ? 0.5 : 1.0);
+          const long long g = cf.off + lin(fi, fj, fk, cf.ny, cf.nz);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) acc[c] += w * (double)ld_val(rf + ((long long)rhs * 3 + c) * ntf + g);
-          }
+          for (int c = 0; c < 3; ++c) acc[c] += w * (double)ld_val(rf + ((long long)rhs * 3 + c) * ntf + g);
         }
       }
     }
@@ -899,7 +919,7 @@ __global__ void k_restrict(const CellDesc* fine, const CellDesc* coarse, const N
 // Trilinear prolongation and correction: xf(n) += sum_I w(n,I) ec(I).
 // Each thread corrects the two fine nodes 2m and 2m+1 of a z row, which share
 // the coarse z nodes m and m+1 (fine 2m = coarse m; fine 2m+1 = mean of m, m+1);
-// x and y weights are uniform along the row.  The pinned node 0 keeps 0.
+// x and y weights are uniform along the row.
 // (All multigrid levels have even fine extents, so pairs never straddle rows.)
 template <typename TF, typename TCo>
 __global__ void k_prolong_add(const CellDesc* __restrict__ fine, const CellDesc* __restrict__ coarse,
@@ -942,7 +962,7 @@ __global__ void k_prolong_add(const CellDesc* __restrict__ fine, const CellDesc*
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       TF* px = xf + ((long long)rhs * 3 + c) * ntf + cf.off + n;
-      if (n != 0) st_val(px, (double)ld_val(px) + a0[c]);
+      st_val(px, (double)ld_val(px) + a0[c]);
       if (n + 1 < u.end) st_val(px + 1, (double)ld_val(px + 1) + a1[c]);
     }
   }
@@ -981,8 +1001,10 @@ __global__ void k_jacobi0(const CellDesc* cells, const NodeUnit* units, const TB
 }
 
 // Dense coarse operator of one cell (one CTA per cell), FP64: A = sum_e kc_e K0(1)
-// scattered to the periodic DOFs; the 3 DOFs of node 0 are replaced by identity
-// rows/columns (pinned).  A is m x m, m = 3 * nodes.
+// scattered to the periodic DOFs, plus the mean diagonal times the projector
+// on the three translations, A's null space (A + a e_c e_c^T / nodes for each
+// component c): on a right-hand side without net force the regular matrix's
+// solution is A's, with no net translation.  A is m x m, m = 3 * nodes.
 template <typename TC>
 __global__ void k_coarse_assemble(const CellDesc* cells, const int* list, const TC* kc,
                                   const double* K0, double* A, const long long* aoff) {
@@ -1007,11 +1029,12 @@ __global__ void k_coarse_assemble(const CellDesc* cells, const int* list, const 
     }
     __syncthreads();
   }
-  for (int t = threadIdx.x; t < m; t += blockDim.x)
-    for (int c = 0; c < 3; ++c) {
-      M[(long long)c * m + t] = (t == c) ? 1.0 : 0.0;
-      M[(long long)t * m + c] = (t == c) ? 1.0 : 0.0;
-    }
+  // mean diagonal: every voxel adds kc_e K0[0] to each of its 8 corners' diagonals
+  double sum = 0.0;
+  for (long long e = 0; e < nn; ++e) sum += (double)kc[cd.off + e];
+  const double a = 8.0 * K0[0] * sum / ((double)nn * (double)nn);
+  for (long long t = threadIdx.x; t < (long long)m * m; t += blockDim.x)
+    if (t / m % 3 == t % m % 3) M[t] += a;
 }
 
 // In-place Cholesky A = L L^T, then A <- A^{-1} (explicit SPD inverse, FP64),
@@ -1155,7 +1178,7 @@ __global__ void k_coarse_solve(const CellDesc* cells, const int* list, const dou
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) {
       const int n = t / 3, c = t % 3;
-      st_val(x + ((long long)rhs * 3 + c) * ntot + cd.off + n, (n == 0) ? 0.0 : s);
+      st_val(x + ((long long)rhs * 3 + c) * ntot + cd.off + n, s);
     }
   }
 }
@@ -1403,6 +1426,18 @@ __global__ void k_param_sum(const int* __restrict__ ptr, const int* __restrict__
 }
 
 
+// Mean load per (cell, load case, component) from k_rhs's sums.
+__global__ void k_rhs_mean(const CellDesc* cells, const int* slot_begin, const int* slot_end, const double* part,
+                           double* mean, int ncells) {
+  FIN_PROLOGUE
+  const double nn = (double)cells[cell].nx * cells[cell].ny * cells[cell].nz;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double v = sum_slots(part, slot_begin[cell], slot_end[cell], rhs, 3, c);
+    if (lead) mean[t * 3 + c] = v / nn;
+  }
+}
+
 __global__ void k_sum_slots(const int* slot_begin, const int* slot_end, const double* part, double* out,
                             int ncells) {
   FIN_PROLOGUE
@@ -1411,8 +1446,9 @@ __global__ void k_sum_slots(const int* slot_begin, const int* slot_end, const do
 }
 
 // Full-cell displacement on (nx+1)(ny+1)(nz+1) nodes for load case I: periodic
-// chi plus the macro-strain affine field, the jump eps (X - X0) on the + faces
-// included (fast_fem/FEM3DFun.cpp:31-56 copyPeriodicU).  Layout [node][3].
+// chi (with node 0 at zero) plus the macro-strain affine field, the jump
+// eps (X - X0) on the + faces included (fast_fem/FEM3DFun.cpp:31-56
+// copyPeriodicU).  Layout [node][3].
 __global__ void k_full_field(const CellDesc* cells, int cell, const double* chi, int I, double* out,
                              long long ntot) {
   const CellDesc cd = cells[cell];
@@ -1432,7 +1468,8 @@ __global__ void k_full_field(const CellDesc* cells, int cell, const double* chi,
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const double aff = eps[c][0] * X[0] + eps[c][1] * X[1] + eps[c][2] * X[2];
-      out[3 * t + c] = chi[((long long)I * 3 + c) * ntot + n0] + aff;
+      const double* x = chi + ((long long)I * 3 + c) * ntot;
+      out[3 * t + c] = x[n0] - x[cd.off] + aff;
     }
   }
 }
@@ -1440,9 +1477,10 @@ __global__ void k_full_field(const CellDesc* cells, int cell, const double* chi,
 }  // namespace femh
 
 namespace femh {
-// [6][3][node] (engine) <-> [6][node][3] (reference layout) for one cell.
+// [6][3][node] (engine) <-> [6][node][3] (reference layout) for one cell;
+// pin (to the reference layout only): every field relative to its node 0.
 template <bool TO_AOS>
-__global__ void k_layout(const double* src, double* dst, long long off, long long nn, long long ntot) {
+__global__ void k_layout(const double* src, double* dst, long long off, long long nn, long long ntot, int pin) {
   const long long total = nn * 18;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -1452,7 +1490,7 @@ __global__ void k_layout(const double* src, double* dst, long long off, long lon
     const int c = (int)(rem - n * 3);
     const long long eng = ((long long)I * 3 + c) * ntot + off + n;   // engine index
     const long long ref = t;                                          // [I][n][c] of this cell
-    if (TO_AOS) dst[ref] = src[eng];
+    if (TO_AOS) dst[ref] = pin ? src[eng] - src[eng - n] : src[eng];
     else dst[eng] = src[ref];
   }
 }

@@ -31,7 +31,7 @@ enum OutMode : int {
   OUT_APPLY_DOT = 1,   // out = K u, partial u . K u
   OUT_JACOBI = 2,      // out = u + omega * D^-1 (b - K u), D point or node-block diagonal
   OUT_JACOBI_DOT = 3,  // same, partial out . b
-  OUT_RESID = 4,       // out = b - K u (pinned node 0 of each cell set to 0)
+  OUT_RESID = 4,       // out = b - K u
 };
 
 template <typename TIn, typename TOut, typename TB, typename TC>
@@ -42,7 +42,7 @@ struct StencilArgs {
   TOut* out;
   const TB* b;
   const TC* kc;          // per voxel c_e * h (level scale folded in)
-  const float* invd;     // per node inverse diagonal (0 at the pinned node)
+  const float* invd;     // per node inverse diagonal
   double* partials;      // [slot][6]
   const CGState* stt;    // per (cell, rhs) state (skip inactive) or nullptr
   long long ntot;        // nodes of the level over all cells
@@ -203,13 +203,12 @@ stencil_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
         if (OUT == OUT_APPLY_DOT) acc += (double)unode[c] * (double)y[c];
       }
     } else {
-      const bool pin = (pg + col0 == 0);
       T dv[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) dv[c] = eb[c] - y[c];
       if (OUT == OUT_RESID) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) st_val(ob + c * st, pin ? (T)0 : dv[c]);
+        for (int c = 0; c < 3; ++c) st_val(ob + c * st, dv[c]);
       } else {
         jacobi_dir<T>(a.binv, cd.off + pg + col0, (T)a.omega * eid, dv);   // point: omega invd folded in
         const T sc = a.binv ? (T)a.omega : (T)1;
@@ -428,13 +427,12 @@ stencil2_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
         if (OUT == OUT_APPLY_DOT) acc += (double)un_[c] * (double)y[c];
       }
     } else {
-      const bool pin = (node == 0);
       T dv[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) dv[c] = ebv[c] - y[c];
       if (OUT == OUT_RESID) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) st_val(ob + c * st, pin ? (T)0 : dv[c]);
+        for (int c = 0; c < 3; ++c) st_val(ob + c * st, dv[c]);
       } else {
         jacobi_dir<T>(a.binv, cd.off + node, (T)a.omega * idv, dv);   // point: omega invd folded in
         const T sc = a.binv ? (T)a.omega : (T)1;
@@ -801,7 +799,6 @@ stencilp_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
         }
       }
     } else {
-      const bool pin = (pg + col0 == 0);
       const f2 wd = p_bc((float)a.omega * eid);
       f2 bd[3];   // node-block Jacobi: B (b - y), both load cases
       if (OUT != OUT_RESID && a.binv) {
@@ -821,8 +818,8 @@ stencilp_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
         const f2 bv = make_float2((float)ebA[c], (float)ebB[c]);
         const f2 d = p_sub(bv, y[c]);
         if (OUT == OUT_RESID) {
-          st_val(ob + c * st, pin ? 0.f : d.x);
-          st_val(ob + c * st + st3, pin ? 0.f : d.y);
+          st_val(ob + c * st, d.x);
+          st_val(ob + c * st + st3, d.y);
         } else {
           const f2 xv = a.binv ? p_fma(p_bc((float)a.omega), bd[c], unode[c]) : p_fma(wd, d, unode[c]);
           st_val(ob + c * st, xv.x);
@@ -1086,7 +1083,6 @@ stencil2p_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
         }
       }
     } else {
-      const bool pin1 = (pg + c1 == 0), pin2 = (pg + c2 == 0);
       const f2 wd = p_mul(p_bc((float)a.omega), id12);
       f2 bd[3];   // node-block Jacobi: B (b - y) of both nodes
       if (OUT != OUT_RESID && a.binv) {
@@ -1099,8 +1095,8 @@ stencil2p_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
         const f2 bv = make_float2((float)eb1[c], (float)eb2[c]);
         const f2 d = p_sub(bv, y[c]);
         if (OUT == OUT_RESID) {
-          if (own1) st_val(ob + c * st + c1, pin1 ? 0.f : d.x);
-          if (own2) st_val(ob + c * st + c2, pin2 ? 0.f : d.y);
+          if (own1) st_val(ob + c * st + c1, d.x);
+          if (own2) st_val(ob + c * st + c2, d.y);
         } else {
           const f2 xv = a.binv ? p_fma(p_bc((float)a.omega), bd[c], u12[c]) : p_fma(wd, d, u12[c]);
           if (own1) st_val(ob + c * st + c1, xv.x);
@@ -1502,7 +1498,6 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
           }
         }
       } else {
-        const bool pin1 = (pg + c1 == 0), pin2 = (pg + c2 == 0);
         const float* Bs = S + oB;
         // rows beyond the tile read stale stage entries: their lanes are not stored
         f2 bv[3], d[3];
@@ -1514,8 +1509,8 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
         if (OUT == OUT_RESID) {
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            if (own1) ob[c * st + c1] = pin1 ? 0.f : d[c].x;
-            if (own2) ob[c * st + c2] = pin2 ? 0.f : d[c].y;
+            if (own1) ob[c * st + c1] = d[c].x;
+            if (own2) ob[c * st + c2] = d[c].y;
           }
         } else {
           const float* Is = S + oI;
@@ -1810,7 +1805,6 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
     const double* Qg = Q + buf * QS;
     double* ob = obase + pg + col;
     const int rb = (r - 1) * nz + z;   // owned row in the b / invd arrays
-    const bool pin = (pg + col == 0);
     const double* Bs = reinterpret_cast<const double*>(S + bB);
     double y[3];
 #pragma unroll
@@ -1824,7 +1818,7 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
       }
     } else if (OUT == OUT_RESID) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) ob[c * st] = pin ? 0.0 : Bs[c * RB * nz + rb] - y[c];
+      for (int c = 0; c < 3; ++c) ob[c * st] = Bs[c * RB * nz + rb] - y[c];
     } else {
       const float* Is = reinterpret_cast<const float*>(S + bI);
       double dv[3];

@@ -22,8 +22,8 @@
  *     upper triangle of its G, fast_fem/FEM3DFun.cpp:163-178; both halves here);
  *   - lower-triangle order of 21-entry outputs: (0,0),(1,0),(1,1),(2,0),...
  *     (the order NumericalCoarseningUsingMultiGrid.cpp:315-324 appends);
- *   - node 0 of every cell is pinned (removes the 3 translations); C^H does not
- *     depend on that choice.
+ *   - displacement fields are reported with node 0 at zero; the solve itself
+ *     leaves the 3 translations free (C^H and the gradients do not depend on them).
  * Threading: one handle = one CUDA stream; calls on one handle are serialised
  * by the caller; different handles are independent.
  * Ownership: inputs and outputs belong to the caller; the handle keeps its own
