@@ -645,7 +645,6 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
       L.d_aoff = upload(ar, aoff, s);
       L.d_A = ar.arr<double>(o);
       L.d_Awork = ar.arr<double>(o);
-      L.d_cstat = ar.arr<int>(L.coarse_list.size());
     }
   }
   // ---- fine-level arrays
@@ -994,26 +993,21 @@ void prepare_operator(femh_handle* H) {
     }
     if (!L.coarse_list.empty()) {
       const unsigned n = (unsigned)L.coarse_list.size();
+      const int T = (L.coarse_maxm + kSweep - 1) / kSweep;
       {
         Prof prof_(H, "k_coarse_assemble", 0.0);
-        k_coarse_assemble<TC><<<n, 256, 0, s>>>(L.d_cells, L.d_coarse_list, (const TC*)L.kc, H->d_K0, L.d_A,
-                                              L.d_aoff);
+        auto fn = k_coarse_assemble<TC>;
+        const size_t sm = sizeof(double) * 3 * L.coarse_maxm;   // up to 108 KB (1536 nodes)
+        if (sm > 48 * 1024)
+          CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        fn<<<dim3(n, (unsigned)L.coarse_maxm / 3), 96, sm, s>>>(L.d_cells, L.d_coarse_list, (const TC*)L.kc, H->d_K0,
+                                                               L.d_A, L.d_Awork, L.d_aoff);
         LAUNCH_CHECK(H);
       }
-      {
-        Prof prof_(H, "k_coarse_factor", 0.0);
-        if (L.coarse_maxm <= kCoarseSmemM) {   // packed triangle in shared memory
-          static bool attr = false;
-          if (!attr) {
-            CK(cudaFuncSetAttribute(k_coarse_factor_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)coarse_factor_smem_bytes(kCoarseSmemM)));
-            attr = true;
-          }
-          k_coarse_factor_smem<<<n, 1024, coarse_factor_smem_bytes(L.coarse_maxm), s>>>(
-              L.d_cells, L.d_coarse_list, L.d_A, L.d_aoff, L.d_cstat);
-        } else {
-          k_coarse_factor<<<n, 256, 0, s>>>(L.d_cells, L.d_coarse_list, L.d_A, L.d_Awork, L.d_aoff, L.d_cstat);
-        }
+      for (int step = 0; step < T; ++step) {
+        Prof prof_(H, "k_coarse_sweep", 0.0);
+        k_coarse_sweep<<<dim3(n, (unsigned)(T * (T + 1) / 2)), 256, 0, s>>>(L.d_cells, L.d_coarse_list, L.d_A,
+                                                                           L.d_Awork, L.d_aoff, step);
         LAUNCH_CHECK(H);
       }
     }

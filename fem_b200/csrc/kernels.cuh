@@ -1000,155 +1000,162 @@ __global__ void k_jacobi0(const CellDesc* cells, const NodeUnit* units, const TB
   }
 }
 
-// Dense coarse operator of one cell (one CTA per cell), FP64: A = sum_e kc_e K0(1)
-// scattered to the periodic DOFs, plus the mean diagonal times the projector
-// on the three translations, A's null space (A + a e_c e_c^T / nodes for each
-// component c): on a right-hand side without net force the regular matrix's
-// solution is A's, with no net translation.  A is m x m, m = 3 * nodes.
+// Dense coarse operator, FP64: A = sum_e kc_e K0(1) scattered to the periodic
+// DOFs, plus the mean diagonal times the projector on the three translations,
+// A's null space (A + a e_c e_c^T / nodes for each component c): on a
+// right-hand side without net force the regular matrix's solution is A's, with
+// no net translation.  A is m x m, m = 3 * nodes.  One 96-thread CTA per (node, cell) owns the
+// node's three rows, gathers its 8 voxels (one after another: a corner pair of
+// two voxels may meet in the same entry) in shared memory and writes the rows
+// once.  A CTA per cell that scattered voxel after voxel took 66 us at 64
+// nodes and 162 us at 105; a row owner needs 8 steps whatever the size (~4 us).
+// Cells whose sweep takes an odd number of block steps start in `work`, so
+// that the last step of every cell writes A (k_coarse_sweep).
+constexpr int kSweep = 32;   // block size of the coarse inversion
 template <typename TC>
-__global__ void k_coarse_assemble(const CellDesc* cells, const int* list, const TC* kc,
-                                  const double* K0, double* A, const long long* aoff) {
+__global__ void __launch_bounds__(96) k_coarse_assemble(const CellDesc* cells, const int* list, const TC* kc,
+                                                        const double* K0, double* A, double* work,
+                                                        const long long* aoff) {
+  extern __shared__ double rows[];   // [3][m]
   const CellDesc cd = cells[list[blockIdx.x]];
-  const long long nn = (long long)cd.nx * cd.ny * cd.nz;
-  const int m = (int)(3 * nn);
-  double* M = A + aoff[blockIdx.x];
-  for (long long t = threadIdx.x; t < (long long)m * m; t += blockDim.x) M[t] = 0.0;
-  __syncthreads();
-  for (long long e = 0; e < nn; ++e) {
-    int i, j, k;
-    node_ijk(e, cd.ny, cd.nz, i, j, k);
-    const double ke = (double)kc[cd.off + e];
-    for (int t = threadIdx.x; t < 576; t += blockDim.x) {
-      const int p = t / 24, q = t % 24;
-      const int ap = p / 3, cp = p % 3, aq = q / 3, cq = q % 3;
-      const long long np = lin(wrap(i + ((ap >> 2) & 1), cd.nx), wrap(j + ((ap >> 1) & 1), cd.ny),
-                               wrap(k + (ap & 1), cd.nz), cd.ny, cd.nz);
-      const long long nq = lin(wrap(i + ((aq >> 2) & 1), cd.nx), wrap(j + ((aq >> 1) & 1), cd.ny),
-                               wrap(k + (aq & 1), cd.nz), cd.ny, cd.nz);
-      M[(3 * np + cp) * m + 3 * nq + cq] += ke * K0[t];
-    }
-    __syncthreads();
-  }
+  const int nn = cd.nx * cd.ny * cd.nz, m = 3 * nn, n = blockIdx.y;
+  if (n >= nn) return;
+  double* M = ((m + kSweep - 1) / kSweep % 2 ? work : A) + aoff[blockIdx.x];
   // mean diagonal: every voxel adds kc_e K0[0] to each of its 8 corners' diagonals
-  double sum = 0.0;
-  for (long long e = 0; e < nn; ++e) sum += (double)kc[cd.off + e];
-  const double a = 8.0 * K0[0] * sum / ((double)nn * (double)nn);
-  for (long long t = threadIdx.x; t < (long long)m * m; t += blockDim.x)
-    if (t / m % 3 == t % m % 3) M[t] += a;
+  // (every CTA adds the same voxels in the same order)
+  double sum[1] = {0.0};
+  for (int e = threadIdx.x; e < nn; e += blockDim.x) sum[0] += (double)kc[cd.off + e];
+  __shared__ double red[32];
+  __shared__ double shift;
+  block_reduce<1>(sum, red);
+  if (threadIdx.x == 0) shift = 8.0 * K0[0] * sum[0] / ((double)nn * (double)nn);
+  __syncthreads();
+  for (int t = threadIdx.x; t < 3 * m; t += blockDim.x) rows[t] = t / m == t % m % 3 ? shift : 0.0;
+  __syncthreads();
+  int i, j, k;
+  node_ijk(n, cd.ny, cd.nz, i, j, k);
+  const int t = threadIdx.x, aq = t / 9, cp = t / 3 % 3, cq = t % 3;   // 72 of the threads: corner, row, column
+  for (int ap = 0; ap < 8; ++ap) {
+    if (t < 72) {
+      const int ei = wrap(i - (ap >> 2 & 1), cd.nx), ej = wrap(j - (ap >> 1 & 1), cd.ny),
+                ek = wrap(k - (ap & 1), cd.nz);
+      const int nq = (int)lin(wrap(ei + (aq >> 2 & 1), cd.nx), wrap(ej + (aq >> 1 & 1), cd.ny),
+                              wrap(ek + (aq & 1), cd.nz), cd.ny, cd.nz);
+      rows[cp * m + 3 * nq + cq] +=
+          (double)kc[cd.off + lin(ei, ej, ek, cd.ny, cd.nz)] * K0[(3 * ap + cp) * 24 + 3 * aq + cq];
+    }
+    __syncthreads();
+  }
+  for (int q = t; q < 3 * m; q += blockDim.x) M[(long long)3 * n * m + q] = rows[q];
 }
 
-// In-place Cholesky A = L L^T, then A <- A^{-1} (explicit SPD inverse, FP64),
-// one CTA per cell.  work holds m*m doubles per cell.  status[cell] = 0 ok,
-// k+1 if pivot k was not positive.
-__global__ void k_coarse_factor(const CellDesc* cells, const int* list, double* A, double* work,
-                                const long long* aoff, int* status) {
+// Explicit inverse of every cell's SPD coarse matrix by symmetric block sweeps
+// (the sweep operator of regression, Goodnight, Am. Stat. 33, 1979, with 32 x
+// 32 blocks): step k replaces, with D = A_kk^-1,
+//   A_kk <- -D,   A_ik <- A_ik D,   A_ij <- A_ij - A_ik D A_kj,
+// and after all block steps the matrix is -A^-1 (the last step stores the
+// negative).  The Cholesky factorisation and column solves that this replaces
+// ran on one CTA per cell, a chain of m pivots each with a pass over the
+// trailing matrix: 1.60 ms at m = 192, 26.3 ms at 315, 150 ms at 600.  Here a
+// step is one launch whose CTAs (one per lower-triangle tile and cell) each
+// invert the 32 x 32 pivot block themselves (32 short pivots in shared memory,
+// the same pivots as Cholesky's) and do the rank-32 update of their tile, so
+// the chain is ceil(m / 32) launches.  Steps go from one buffer to the other:
+// tiles read the pivot row and column of the previous step while the same
+// launch rewrites them.  Tiles i > j are stored twice, so the inverse is
+// symmetric to the last bit, which the V-cycle needs to be a symmetric
+// preconditioner.  A pivot that is not positive (a floating part of a
+// zero-stiffness cell) is replaced by 1e-300.
+__global__ void __launch_bounds__(256) k_coarse_sweep(const CellDesc* cells, const int* list, double* A, double* work,
+                                                      const long long* aoff, int step) {
   const CellDesc cd = cells[list[blockIdx.x]];
-  const int m = 3 * cd.nx * cd.ny * cd.nz;
-  double* L = A + aoff[blockIdx.x];
-  double* X = work + aoff[blockIdx.x];
-  __shared__ int bad;
-  if (threadIdx.x == 0) bad = 0;
-  __syncthreads();
-  for (int k = 0; k < m; ++k) {
-    if (threadIdx.x == 0) {
-      const double d = L[(long long)k * m + k];
-      if (!(d > 0.0) && !bad) bad = k + 1;
-      L[(long long)k * m + k] = sqrt(fmax(d, 1e-300));
-    }
-    __syncthreads();
-    const double dk = L[(long long)k * m + k];
-    for (int i = k + 1 + threadIdx.x; i < m; i += blockDim.x) L[(long long)i * m + k] /= dk;
-    __syncthreads();
-    for (long long t = threadIdx.x; t < (long long)(m - k - 1) * (m - k - 1); t += blockDim.x) {
-      const int i = k + 1 + (int)(t / (m - k - 1)), j = k + 1 + (int)(t % (m - k - 1));
-      if (j <= i) L[(long long)i * m + j] -= L[(long long)i * m + k] * L[(long long)j * m + k];
-    }
-    __syncthreads();
-  }
-  // X = A^{-1}: solve L L^T X = I column by column (threads over columns)
-  for (int col = threadIdx.x; col < m; col += blockDim.x) {
-    for (int i = 0; i < m; ++i) {   // forward: L y = e_col
-      double s = (i == col) ? 1.0 : 0.0;
-      for (int j = 0; j < i; ++j) s -= L[(long long)i * m + j] * X[(long long)j * m + col];
-      X[(long long)i * m + col] = s / L[(long long)i * m + i];
-    }
-    for (int i = m - 1; i >= 0; --i) {   // backward: L^T x = y
-      double s = X[(long long)i * m + col];
-      for (int j = i + 1; j < m; ++j) s -= L[(long long)j * m + i] * X[(long long)j * m + col];
-      X[(long long)i * m + col] = s / L[(long long)i * m + i];
-    }
-  }
-  __syncthreads();
-  for (long long t = threadIdx.x; t < (long long)m * m; t += blockDim.x) L[t] = X[t];
-  if (threadIdx.x == 0) status[blockIdx.x] = bad;
-}
-
-// The same factorisation and inverse for coarse systems of m <= kCoarseSmemM
-// unknowns (3 x 64 nodes): the lower triangle of A packed in shared memory
-// (row i at i(i+1)/2), right-looking Cholesky in place (one warp per trailing
-// row, lanes over its columns), then A^{-1} column by column, one warp per
-// column: forward L y = e_c from row c on (y = 0 above), backward L^T x = y,
-// each row's dot product split over the lanes.  Written over A.
-constexpr int kCoarseSmemM = 192;
-inline size_t coarse_factor_smem_bytes(int m) {
-  return sizeof(double) * ((size_t)m * (m + 1) / 2 + 32 * (size_t)m);
-}
-__global__ void __launch_bounds__(1024) k_coarse_factor_smem(const CellDesc* cells, const int* list, double* A,
-                                                             const long long* aoff, int* status) {
-  extern __shared__ double csm[];
-  const CellDesc cd = cells[list[blockIdx.x]];
-  const int m = 3 * cd.nx * cd.ny * cd.nz;
-  double* Ag = A + aoff[blockIdx.x];
-  double* Lp = csm;                               // packed lower triangle
-  double* Yw = csm + (size_t)m * (m + 1) / 2;     // [32 warps][m] column buffers
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  auto P = [](int i, int j) { return i * (i + 1) / 2 + j; };   // j <= i
-  __shared__ int bad;
-  if (tid == 0) bad = 0;
-  for (int i = warp; i < m; i += nw)
-    for (int j = lane; j <= i; j += 32) Lp[P(i, j)] = Ag[(long long)i * m + j];
-  __syncthreads();
-  for (int k = 0; k < m; ++k) {
-    if (tid == 0) {
-      const double d = Lp[P(k, k)];
-      if (!(d > 0.0) && !bad) bad = k + 1;
-      Lp[P(k, k)] = sqrt(fmax(d, 1e-300));
-    }
-    __syncthreads();
-    const double dk = Lp[P(k, k)];
-    for (int i = k + 1 + tid; i < m; i += nt) Lp[P(i, k)] /= dk;
-    __syncthreads();
-    for (int i = k + 1 + warp; i < m; i += nw) {
-      const double lik = Lp[P(i, k)];
-      for (int j = k + 1 + lane; j <= i; j += 32) Lp[P(i, j)] -= lik * Lp[P(j, k)];
-    }
-    __syncthreads();
-  }
-  double* y = Yw + (size_t)warp * m;
-  for (int c = warp; c < m; c += nw) {
-    for (int i = lane; i < c; i += 32) y[i] = 0.0;
-    __syncwarp();
-    for (int i = c; i < m; ++i) {   // forward: L y = e_c
-      double sacc = 0.0;
-      for (int j = c + lane; j < i; j += 32) sacc += Lp[P(i, j)] * y[j];
+  const int m = 3 * cd.nx * cd.ny * cd.nz, T = (m + kSweep - 1) / kSweep;
+  if (step >= T) return;
+  // lower-triangle tile (ti, tj) of this CTA
+  int ti = (int)((sqrtf(8.f * blockIdx.y + 1.f) - 1.f) * 0.5f);
+  while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.y) ++ti;
+  while (ti * (ti + 1) / 2 > (int)blockIdx.y) --ti;
+  const int tj = (int)blockIdx.y - ti * (ti + 1) / 2;
+  if (ti >= T) return;
+  const bool in_work = (T - step) % 2 != 0;
+  const double* src = (in_work ? work : A) + aoff[blockIdx.x];
+  double* dst = (in_work ? A : work) + aoff[blockIdx.x];
+  __shared__ double D[kSweep][kSweep + 1], P[kSweep][kSweep + 1], Q[kSweep][kSweep + 1], U[kSweep][kSweep + 1];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;   // tile column, first of 4 rows (stride 8)
+  auto at = [&](int bi, int bj, int r) -> double {   // entry (r, x) of tile (bi, bj), the identity outside
+    const int gi = bi * kSweep + r, gj = bj * kSweep + x;
+    return gi < m && gj < m ? src[(long long)gi * m + gj] : (bi == bj && r == x ? 1.0 : 0.0);
+  };
+  double a[4];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
-      if (lane == 0) y[i] = ((i == c ? 1.0 : 0.0) - sacc) / Lp[P(i, i)];
-      __syncwarp();
-    }
-    for (int i = m - 1; i >= 0; --i) {   // backward: L^T x = y
-      double sacc = 0.0;
-      for (int j = i + 1 + lane; j < m; j += 32) sacc += Lp[P(j, i)] * y[j];
+  for (int q = 0; q < 4; ++q) {
+    const int r = y + 8 * q;
+    D[r][x] = at(step, step, r);
+    P[r][x] = at(ti, step, r);      // A_ik
+    Q[r][x] = at(tj, step, r);      // A_jk = A_kj^T
+    a[q] = at(ti, tj, r);
+  }
+  // D <- A_kk^-1: scalar sweeps, one pivot at a time, in place
+  for (int p = 0; p < kSweep; ++p) {
+    __syncthreads();
+    double d = D[p][p];
+    d = 1.0 / (d > 0.0 ? d : 1e-300);
+    const double cx = D[p][x];
+    double v[4];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
-      if (lane == 0) y[i] = (y[i] - sacc) / Lp[P(i, i)];
-      __syncwarp();
+    for (int q = 0; q < 4; ++q) {
+      const int r = y + 8 * q;
+      const double cr = D[r][p];
+      v[q] = r == p ? (x == p ? -d : cx * d) : (x == p ? cr * d : D[r][x] - cr * d * cx);
     }
-    for (int i = lane; i < m; i += 32) Ag[(long long)i * m + c] = y[i];
-    __syncwarp();
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) D[y + 8 * q][x] = v[q];
   }
   __syncthreads();
-  if (tid == 0) status[blockIdx.x] = bad;
+  // U = A_ik D (D holds -A_kk^-1)
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = y + 8 * q;
+    double u = 0.0;
+#pragma unroll 8
+    for (int p = 0; p < kSweep; ++p) u -= P[r][p] * D[p][x];
+    U[r][x] = u;
+  }
+  __syncthreads();
+  double v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = y + 8 * q;
+    if (ti == step && tj == step) {
+      v[q] = r >= x ? D[r][x] : D[x][r];   // -D
+    } else if (tj == step) {
+      v[q] = U[r][x];                      // A_ik D
+    } else if (ti == step) {               // (A_jk D)^T: row r of the pivot block, column x of tile j
+      double u = 0.0;
+#pragma unroll 8
+      for (int p = 0; p < kSweep; ++p) u -= Q[x][p] * D[p][r];
+      v[q] = u;
+    } else {
+      double u = a[q];
+#pragma unroll 8
+      for (int p = 0; p < kSweep; ++p) u -= U[r][p] * Q[x][p];
+      v[q] = u;
+    }
+    if (step == T - 1) v[q] = -v[q];
+  }
+  __syncthreads();   // P is free: the tile on its way to the mirrored store
+#pragma unroll
+  for (int q = 0; q < 4; ++q) P[y + 8 * q][x] = v[q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = y + 8 * q;
+    const int gi = ti * kSweep + r, gj = tj * kSweep + x;
+    if (gi < m && gj < m && gi >= gj) dst[(long long)gi * m + gj] = P[r][x];
+    const int hi = tj * kSweep + r, hj = ti * kSweep + x;   // mirrored entry
+    if (hi < m && hj < m && hj > hi) dst[(long long)hi * m + hj] = P[x][r];
+  }
 }
 
 // Coarse solve e = A^{-1} b for one (cell, rhs) per CTA (A^{-1} symmetric).

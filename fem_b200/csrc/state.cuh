@@ -124,7 +124,6 @@ struct Level {
   long long* d_aoff = nullptr;
   double* d_A = nullptr;
   double* d_Awork = nullptr;
-  int* d_cstat = nullptr;
   int coarse_maxm = 0;
   void* kc = nullptr;     // TC
   float* invd = nullptr;
