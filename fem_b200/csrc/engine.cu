@@ -498,6 +498,7 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
   if (H->shape_key == shapes && H->h_key == hs && H->prec_key == c.precision && H->solver_key == c.solver &&
       H->bf16_key == c.store_bf16)
     return;
+  release_loops(H);
   H->setup.release();
   release_stage(H);
   H->levels.clear();
@@ -1290,6 +1291,8 @@ void pcg_iteration(femh_handle* H, const typename PR::K* kcg, bool blk) {
   }
 }
 
+template <class PR> inline char prec_tag = 0;   // its address names the precision combination
+
 // PCG on K x = scale*b for every (cell, rhs) whose state is active.
 // warm: x already holds the starting iterate and b is its residual; the
 // relative residual is measured against ||b_orig||^2 in H->d_nrm.
@@ -1387,13 +1390,28 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
   // WHILE node repeats `chunk` captured iterations while k_while_cond finds
   // live cells (and, for a batch, more than half of the listed ones); the host
   // wakes only to compact a batch's unit lists or at the end.
+  // The loop over all cells is captured once per set-up (LoopGraph): its
+  // launches depend on the set-up and on the key below alone.  A batch's
+  // compacted loops are captured each time.
   cudaGraphExec_t exec = nullptr;
+  bool kept = false;             // exec belongs to H->loops
   long long graph_kernels = 0;   // kernels of one pass of the loop body
   int listed = nc;               // cells covered by the current unit lists
   const int limit = max_iter + chunk;
   CK(cudaMemsetAsync(H->d_loop, 0, sizeof(int), s));
   auto capture = [&]() {
     if (!(c.graph_chunk > 0 && !H->prof)) return;
+    const bool all_cells = listed == nc;
+    if (all_cells)
+      for (auto& g : H->loops)
+        if (g.prec == &prec_tag<PR> && g.kcg == kcg && g.limit == limit && g.chunk == chunk && g.block == blk &&
+            g.persist == H->persist_ok) {
+          exec = g.exec;
+          graph_kernels = g.kernels;
+          kept = true;
+          return;
+        }
+    kept = false;
     cudaGraph_t g = nullptr;
     CK(cudaGraphCreate(&g, 0));
     cudaGraphConditionalHandle cond;
@@ -1436,7 +1454,16 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
     }
     const cudaError_t ei = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
+    if (ei != cudaSuccess) exec = nullptr;
     CK(ei);
+    if (all_cells) {
+      H->loops.push_back({&prec_tag<PR>, kcg, limit, chunk, blk, H->persist_ok, exec, graph_kernels});
+      kept = true;
+    }
+  };
+  auto drop = [&]() {
+    if (exec && !kept) cudaGraphExecDestroy(exec);
+    exec = nullptr;
   };
   // batch compaction bookkeeping
   std::vector<FullLists> full;
@@ -1485,19 +1512,16 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
         }
         for (size_t l = 0; l < H->levels.size(); ++l) set_units(H, H->levels[l], full[l], &keep);
         listed = alive;
-        if (exec) {
-          CK(cudaGraphExecDestroy(exec));
-          exec = nullptr;
-        }
+        drop();
         capture();
       }
     }
   } catch (...) {
-    if (exec) cudaGraphExecDestroy(exec);
+    drop();
     restore();
     throw;
   }
-  if (exec) CK(cudaGraphExecDestroy(exec));
+  drop();
   restore();
   for (int t = 0; t < nc * kNumRhs; ++t) iters_out[t] += H->state[t].iters;
   if (blk) {   // cells whose block step matrices turned indefinite: one load case at a time
@@ -1906,6 +1930,7 @@ femh_status femh_destroy(femh_handle* H) {
   if (!H) return FEMH_E_ARG;
   cudaSetDevice(H->device);
   if (H->stream) cudaStreamSynchronize(H->stream);
+  release_loops(H);
   H->setup.release();
   release_stage(H);
   H->perm.release();

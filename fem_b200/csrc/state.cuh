@@ -209,6 +209,18 @@ struct femh_handle {
   // solves of defect correction finish their load cases at different times
   // (the CTAs of a finished one would idle), so they run one CTA per unit
   bool persist_ok = true;
+  // captured CG loops (pcg), kept until the set-up they run on goes: a capture
+  // and its instantiation cost the host milliseconds, as much as a small solve.
+  // At most one entry per loop a configuration uses (block, one case at a time).
+  struct LoopGraph {
+    const void* prec;   // precision tag of pcg<PR>
+    const void* kcg;
+    int limit, chunk;
+    bool block, persist;
+    cudaGraphExec_t exec;
+    long long kernels;  // kernels of one pass of the loop body
+  };
+  std::vector<LoopGraph> loops;
   int* d_loop = nullptr;         // CG iterations run on the device in the current solve (WHILE-node count)
   int* d_err = nullptr;   // [0] set by a stencil kernel whose bounded wait ran out,
                           // [1] by k_coef on a NaN, infinite or negative density
@@ -273,6 +285,11 @@ struct Prof {
     }
   }
 };
+
+inline void release_loops(femh_handle* H) {
+  for (auto& g : H->loops) cudaGraphExecDestroy(g.exec);
+  H->loops.clear();
+}
 
 inline void prof_resolve(femh_handle* H) {
   if (H->pend.empty()) return;
