@@ -299,10 +299,11 @@ MatLaw make_law(const femh_config& c) {
   return m;
 }
 
-// Stencil work units of one cell: tiles of up to R-1 rows, x-chunks of len.
-void add_stencil_units(std::vector<StencilUnit>& out, int cellidx, const CellDesc& cd, int NT,
+// Stencil work units of one cell: tiles of up to R-1 rows, x-chunks of len
+// (R = NT / pitch thread rows).
+void add_stencil_units(std::vector<StencilUnit>& out, int cellidx, const CellDesc& cd, int NT, int pitch,
                        int& slot, int chunk_req = 0, int variant = 2) {
-  const int R = NT / cd.nz;
+  const int R = NT / pitch;
   const bool two_rows = variant == 2 || variant == 4 || variant == 5 || variant == 7;
   const int maxrows = std::max(1, std::min(two_rows ? 2 * R - 1 : R - 1, cd.ny));
   const int ntiles = (cd.ny + maxrows - 1) / maxrows;
@@ -333,9 +334,19 @@ void add_node_units(std::vector<NodeUnit>& out, int cellidx, long long nn, int& 
 
 template <typename T> size_t esize() { return sizeof(T); }
 
-// Threads per CTA that a cell's stencil units are cut for.
+// Whether a variant runs the staged kernels on a level (else stencil() takes
+// the unstaged kernel of the same tiles).
+bool staged_on(const Level& L, int variant) {
+  return variant == 6 ? L.bulk_ok64 : (variant == 5 || variant == 7) && L.bulk_ok;
+}
+
+// Threads per CTA, and row pitch across them, that a cell's stencil units are cut for.
 int cell_nt(const Level& L, const CellDesc& cd, int variant) {
+  if (staged_on(L, variant)) return variant == 6 ? stage_nt64(stage_class(cd.nz)) : kStageNT32;
   return L.grouped ? variant_nt(spec_nt(cd.nz), cd.nz, variant) : variant_nt(L.NT, L.maxnz, variant);
+}
+int cell_pitch(const Level& L, const CellDesc& cd, int variant) {
+  return staged_on(L, variant) ? stage_class(cd.nz) : cd.nz;
 }
 
 // On grouped levels: sort a unit list by z extent (stable, so each cell's
@@ -581,20 +592,20 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
       }
       L.grouped = L.nz_spec == 0 && all_spec && !same;
     }
-    // bulk-copy staging needs compile-time z extents with 16-byte rows (all in
-    // the compile-time set are multiples of 4); a tile never has more rows than
-    // its cell, so each staged array takes at most three row segments (20
-    // copies per stage at most, within warp 0's lanes)
-    L.bulk_ok = (L.nz_spec > 0 || L.grouped) && L.maxnz <= 128;
-    L.bulk_ok64 = L.nz_spec > 0 || L.grouped;
+    // bulk-copy staging needs one z extent (or, grouped, one per launch) with a row pitch
+    bool same_nz = true;
+    for (auto& cd : L.cells) same_nz = same_nz && cd.nz == L.cells[0].nz;
+    L.bulk_ok64 = (same_nz && stage_class(L.maxnz) > 0) || L.grouped;
+    L.bulk_ok = L.bulk_ok64 && (L.grouped ? L.maxnz <= 128 : L.maxnz <= 192);
     if (c.stencil_variant > 0) L.variant = c.stencil_variant;
     if (L.variant == 7 && L.grouped) L.variant = 5;   // persistent CTAs need one z extent
     if ((L.variant == 5 || L.variant == 7) && !L.bulk_ok) L.variant = 4;
+    if (L.variant == 6 && !L.bulk_ok64) L.variant = 2;
     int ss = 0, sn = 0;
     for (int ci = 0; ci < (int)L.cells.size(); ++ci) {
       const CellDesc& cd = L.cells[ci];
       L.su_sb.push_back(ss);
-      add_stencil_units(L.all.su, ci, cd, cell_nt(L, cd, L.variant), ss, 0, L.variant);
+      add_stencil_units(L.all.su, ci, cd, cell_nt(L, cd, L.variant), cell_pitch(L, cd, L.variant), ss, 0, L.variant);
       L.su_se.push_back(ss);
       L.nu_sb.push_back(sn);
       add_node_units(L.all.nu, ci, (long long)cd.nx * cd.ny * cd.nz, sn, l == 0 ? 2048 : 256);
@@ -762,7 +773,8 @@ void build_stencil_units(femh_handle* H, Level& L, int chunk) {
   int ss = 0;
   for (int ci = 0; ci < (int)L.cells.size(); ++ci) {
     L.su_sb.push_back(ss);
-    add_stencil_units(L.all.su, ci, L.cells[ci], cell_nt(L, L.cells[ci], L.variant), ss, chunk, L.variant);
+    add_stencil_units(L.all.su, ci, L.cells[ci], cell_nt(L, L.cells[ci], L.variant),
+                      cell_pitch(L, L.cells[ci], L.variant), ss, chunk, L.variant);
     L.su_se.push_back(ss);
   }
   group_units(L, L.all.su, L.gall, true);
@@ -789,7 +801,8 @@ void build_stencil_units64(femh_handle* H, Level& L, int chunk, int variant) {
   int ss = 0;
   for (int ci = 0; ci < (int)L.cells.size(); ++ci) {
     L.su64_sb.push_back(ss);
-    add_stencil_units(L.su64, ci, L.cells[ci], cell_nt(L, L.cells[ci], variant), ss, chunk, variant);
+    add_stencil_units(L.su64, ci, L.cells[ci], cell_nt(L, L.cells[ci], variant), cell_pitch(L, L.cells[ci], variant),
+                      ss, chunk, variant);
     L.su64_se.push_back(ss);
   }
   group_units(L, L.su64, L.g64, true);

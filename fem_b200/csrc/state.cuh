@@ -100,7 +100,7 @@ struct Level {
   int nz_spec = 0;   // > 0: every cell of the level has this z extent (specialised kernel)
   int chunk = 0;     // x-chunk length of the stencil units (0 = heuristic), set by the autotuner
   int variant = 2;   // stencil kernel (femh_config::stencil_variant numbering)
-  bool bulk_ok = false;     // the bulk-copy staged FP32 kernel (variant 5) can run on this level
+  bool bulk_ok = false;     // the bulk-copy staged FP32 kernel (variants 5, 7) can run on this level
   bool bulk_ok64 = false;   // the bulk-copy staged FP64 kernel (variant 6) can run on this level
   // cells of several z extents, each one with a compile-time kernel (a batch
   // of uneven cells): the unit lists are sorted by z extent and each extent
@@ -318,6 +318,28 @@ inline int variant_nt(int level_nt, int maxnz, int variant) {
 // z extents with compile-time kernels, and their threads per CTA.
 inline bool spec_nz(int nz) { return nz == 16 || nz == 24 || nz == 32 || nz == 48 || nz == 64 || nz == 128 || nz == 256; }
 inline int spec_nt(int nz) { return (nz == 24 || nz == 48) ? 480 : 512; }
+
+// Row pitch of the staged kernels (variants 5 to 7) for a z extent: the
+// smallest class that holds it, 0 if there is none.  Rows are copied in bulk,
+// so extents are multiples of 4 (16 bytes); between the classes a CTA's lanes
+// beyond nz idle (at most 31% of them from 36 on).  FP32 sweep, ms, best
+// unstaged -> staged: 192^3 1.27 -> 0.65, 160^3 0.61 -> 0.49, 112^3 0.236 ->
+// 0.163, 96^3 0.139 -> 0.085, 80^3 0.077 -> 0.065; FP64 apply 192^3 2.66 ->
+// 1.33, 96^3 0.205 -> 0.125.  At 56 and 40 the two are even, and the autotuner
+// times both wherever the staged kernels are eligible.  Below 36 only the
+// classes themselves: the row copies would shrink to 48-112 bytes, over a
+// hundred a step, on levels that the other kernels finish in microseconds.
+inline int stage_class(int nz) {
+  if (nz % 4 != 0) return 0;
+  for (int c : {16, 24, 32, 48, 64, 96, 128, 192, 256})
+    if (nz <= c) return nz == c || nz >= 36 ? c : 0;
+  return 0;
+}
+constexpr int kStageNT32 = 384;   // variants 5, 7: 24 to 2 thread rows
+// variant 6: threads a multiple of the pitch; at 192 two thread rows of which
+// one is the halo (384 threads: 192^3 apply 1.33 ms; three rows of 576 threads
+// hold only 96 registers each and spill: 1.70 ms; unstaged 2.66 ms)
+constexpr int stage_nt64(int c) { return c == 192 ? 384 : (c == 24 || c == 48 || c == 96) ? 480 : 512; }
 
 // One stencil launch set over a level (all cells, or those that are smoothed
 // there).  T = arithmetic type; in/out/b storage types as given.

@@ -1315,15 +1315,37 @@ __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned
 // per unit (written when a unit's last node plane is gathered), so results
 // are the same bits as one CTA per unit.  Stage g of a stream uses ring slot
 // (gbase + g) % kBulkSlots, gbase = stages of the CTA's earlier streams.
+// NZ is the pitch of a row in shared memory and across the threads, a
+// compile-time class (stage_class) at least as long as the cell's rows: only
+// the copies and the global offsets know nz.  A cell with nz == NZ copies
+// row segments (at most ny rows each, so three per array: 20 copies per stage
+// from warp 0's lanes); any other copies row by row, one copy per thread
+// (bulk_rows), and its threads z >= nz idle (figures at stage_class).
 // Requirements (checked by the host): nz % 4 == 0 on every cell, 16-byte
-// aligned arrays.  A tile has at most ny rows, so an array spans at most three
-// row segments: at most 20 copies per stage, one per lane of warp 0.
+// aligned arrays.
 constexpr int kBulkSlots = 4;
+
+// Row-by-row staging: copy number idx of a stage made of NA arrays, array k
+// with n[k] rows.  Returns the array and sets the row, or -1 past the last.
+// (Copies are dealt out over the warps: a warp issues its lanes' copies one
+// after another.)
+template <int NA>
+__device__ __forceinline__ int bulk_rows(int idx, const int (&n)[NA], int& row) {
+#pragma unroll
+  for (int k = 0; k < NA; ++k) {
+    if (idx < n[k]) {
+      row = idx;
+      return k;
+    }
+    idx -= n[k];
+  }
+  return -1;
+}
 
 template <int NT, int OUT, int NZ>
 __global__ void __launch_bounds__(NT, 1)
 stencil2b_kernel(StencilArgs<float, float, float, float> a) {
-  static_assert(NZ > 0 && NZ % 4 == 0, "staged rows need a compile-time z extent, multiple of 4");
+  static_assert(NZ > 0 && NZ % 4 == 0 && NT % NZ == 0, "staged rows need a compile-time pitch, multiple of 4");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int rhs = blockIdx.y;
   int kb = blockIdx.x, ke = blockIdx.x + 1;   // units of this CTA: [kb, ke)
@@ -1331,27 +1353,28 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
     kb = a.cta_units[blockIdx.x];
     ke = a.cta_units[blockIdx.x + 1];
   }
-  constexpr int nz = NZ;
+  if (kb >= ke) return;
   constexpr int TR = NT / NZ;
+  const int nz = a.cells[a.units[kb].cell].nz;   // the same for every cell of the launch
   const int tid = threadIdx.x;
-  const int t = tid / nz, z = tid - t * nz;
+  const int t = tid / NZ, z = tid - t * NZ;
   const int zp = (z + 1 == nz) ? 0 : z + 1;
   const int zm = (z == 0) ? nz - 1 : z - 1;
 
   constexpr int RB = 2 * TR - 1, NRU = RB + 3, NRK = RB + 2;
-  // stage layout (floats): U[3][NRU][nz], KC[NRK][nz], B[3][RB][nz], I[RB][nz][6]
+  // stage layout (floats): U[3][NRU][NZ], KC[NRK][NZ], B[3][RB][NZ], I[RB][NZ][6]
   // (invd rows, or the node-block inverses [6] of a block sweep)
   constexpr int oK = 3 * NRU * NZ, oB = oK + NRK * NZ, oI = oB + 3 * RB * NZ;
   constexpr int SS = (oI + 6 * RB * NZ + 3) & ~3;
-  constexpr int PS = TR * 3 * nz;
+  constexpr int PS = TR * 3 * NZ;
   float* stg = reinterpret_cast<float*>(smem_raw);
-  f2* QAB = reinterpret_cast<f2*>(stg + kBulkSlots * SS);   // [2][TR][3][nz]
+  f2* QAB = reinterpret_cast<f2*>(stg + kBulkSlots * SS);   // [2][TR][3][NZ]
   f2* QCD = QAB + 2 * PS;
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(QCD + 2 * PS);
   double* red = reinterpret_cast<double*>(bars + kBulkSlots);
   __shared__ int abort_flag;
-  const int pt = t * 3 * nz;
-  const int pa = (t + 1 < TR ? t + 1 : t) * 3 * nz;
+  const int pt = t * 3 * NZ;
+  const int pa = (t + 1 < TR ? t + 1 : t) * 3 * NZ;
   const long long st = a.ntot;
 
   if (tid == 0) {
@@ -1378,7 +1401,7 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
     }
     const int nx = cd.nx, ny = cd.ny;
     const int rows = un.rows;
-    const bool live = t < TR && 2 * t <= rows;
+    const bool live = t < TR && 2 * t <= rows && z < nz;
     const bool own1 = live && 2 * t < rows;
     const bool own2 = live && 2 * t + 1 < rows;
     auto wrapy = [&](int j) { j %= ny; return j < 0 ? j + ny : j; };
@@ -1387,42 +1410,67 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
     const int c1 = n1 * nz + z, c2 = n2 * nz + z;
     float* obase = a.out + (long long)rhs * 3 * st + cd.off;
 
+    // this thread's copy of every stage (bytes == 0: none)
     const char* src_base = nullptr;
     int plane_lag = 0, src_off = 0, dst_off = 0, bytes = 0, esz = 4;
     unsigned tx_total = 0;
-    if (tid < 32) {
-      int idx = 0;
-      // es: bytes per node of the array (4, or 24 for the node blocks)
-      auto seg = [&](const float* base, int lag, int row0, int nrows, int dst, int es = 4) {
-        int done = 0;
-        while (done < nrows) {
-          const int r0 = wrapy(row0 + done);
-          const int n = min(nrows - done, ny - r0);
-          if (idx == tid) {
-            src_base = reinterpret_cast<const char*>(base);
-            plane_lag = lag;
-            esz = es;
-            src_off = r0 * nz;
-            dst_off = dst + done * nz * (es / 4);
-            bytes = n * nz * es;
+    const bool sweep = OUT == OUT_JACOBI || OUT == OUT_JACOBI_DOT;
+    const int esI = a.binv ? 24 : 4;   // bytes per node of the inverse diagonals
+    if (nz == NZ) {
+      if (tid < 32) {
+        int idx = 0;
+        // es: bytes per node of the array (4, or 24 for the node blocks)
+        auto seg = [&](const float* base, int lag, int row0, int nrows, int dst, int es = 4) {
+          int done = 0;
+          while (done < nrows) {
+            const int r0 = wrapy(row0 + done);
+            const int n = min(nrows - done, ny - r0);
+            if (idx == tid) {
+              src_base = reinterpret_cast<const char*>(base);
+              plane_lag = lag;
+              esz = es;
+              src_off = r0 * NZ;
+              dst_off = dst + done * NZ * (es / 4);
+              bytes = n * NZ * es;
+            }
+            tx_total += (unsigned)(n * NZ * es);
+            ++idx;
+            done += n;
           }
-          tx_total += (unsigned)(n * nz * es);
-          ++idx;
-          done += n;
-        }
-      };
-      for (int c = 0; c < 3; ++c)
-        seg(a.u + ((long long)rhs * 3 + c) * st + cd.off, 1, un.j0 - 1, rows + 3, c * NRU * nz);
-      seg(a.kc + cd.off, 0, un.j0 - 1, rows + 2, oK);
-      if (OUT >= OUT_JACOBI) {
+        };
         for (int c = 0; c < 3; ++c)
-          seg(a.b + ((long long)rhs * 3 + c) * st + cd.off, -1, un.j0, rows, oB + c * RB * nz);
-        if (OUT != OUT_RESID) {
-          if (a.binv) seg(a.binv + 6 * cd.off, -1, un.j0, rows, oI, 24);
-          else seg(a.invd + cd.off, -1, un.j0, rows, oI);
+          seg(a.u + ((long long)rhs * 3 + c) * st + cd.off, 1, un.j0 - 1, rows + 3, c * NRU * NZ);
+        seg(a.kc + cd.off, 0, un.j0 - 1, rows + 2, oK);
+        if (OUT >= OUT_JACOBI) {
+          for (int c = 0; c < 3; ++c)
+            seg(a.b + ((long long)rhs * 3 + c) * st + cd.off, -1, un.j0, rows, oB + c * RB * NZ);
+          if (sweep) seg(a.binv ? a.binv + 6 * cd.off : a.invd + cd.off, -1, un.j0, rows, oI, esI);
         }
       }
+    } else {
+      const int n[8] = {rows + 3, rows + 3, rows + 3, rows + 2, OUT >= OUT_JACOBI ? rows : 0,
+                        OUT >= OUT_JACOBI ? rows : 0, OUT >= OUT_JACOBI ? rows : 0, sweep ? rows : 0};
+      int row = 0;
+      const int k8 = bulk_rows<8>((tid & 31) * (NT / 32) + (tid >> 5), n, row);
+      if (k8 >= 0) {
+        const int c = k8 < 3 ? k8 : k8 - 4;   // component of a u or b row
+        const float* base = k8 < 3    ? a.u + ((long long)rhs * 3 + c) * st
+                            : k8 == 3 ? a.kc
+                            : k8 < 7  ? a.b + ((long long)rhs * 3 + c) * st
+                            : a.binv  ? a.binv + 5 * cd.off
+                                      : a.invd;
+        src_base = reinterpret_cast<const char*>(base + cd.off);
+        plane_lag = k8 < 3 ? 1 : k8 == 3 ? 0 : -1;
+        esz = k8 == 7 ? esI : 4;
+        src_off = wrapy(un.j0 - (k8 < 4 ? 1 : 0) + row) * nz;
+        dst_off = k8 < 3 ? (c * NRU + row) * NZ : k8 == 3 ? oK + row * NZ : k8 < 7 ? oB + (c * RB + row) * NZ
+                                                                             : oI + row * NZ * (esI / 4);
+        bytes = nz * esz;
+      }
+      tx_total = (unsigned)(nz * 4) * (unsigned)(n[0] + n[1] + n[2] + n[3] + n[4] + n[5] + n[6]) +
+                 (unsigned)(nz * esI) * (unsigned)n[7];
     }
+    const bool issuer = tid == 0 || bytes > 0;
     int pl_next = ((un.i0 - 2 + plane_lag) % nx + nx) % nx;
     int issued = 0;
     auto issue = [&](int g) {
@@ -1430,18 +1478,17 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
       const unsigned gg = gbase + (unsigned)g;
       const int slot = (int)(gg % kBulkSlots);
       const unsigned bar = smem_addr(bars + slot);
-      if (tid == 0) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(bar, tx_total);
-      }
-      __syncwarp();
+      // (a copy may complete before tid 0's arrival announces its bytes: the
+      // phase still waits for that arrival)
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      if (tid == 0) mbar_expect_tx(bar, tx_total);
       if (bytes > 0)
         bulk_g2s(smem_addr(stg + slot * SS + dst_off),
                  src_base + (long long)esz * ((long long)pl_next * plane + src_off), (unsigned)bytes, bar);
       if (++pl_next == nx) pl_next = 0;
     };
     const int G = len + 3;
-    if (tid < 32)
+    if (issuer)
       for (int g = 0; g < kBulkSlots && g < G; ++g) issue(g);
     int waited = 0;
     auto wait_stage = [&](int g) {
@@ -1465,10 +1512,10 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
     auto patch = [&](const float* U, f2 (&h)[3][4], f2 (&mine)[3]) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const float* Uc = U + c * NRU * nz;
-        const int r0 = (2 * t) * nz;
-        mine[c] = make_float2(Uc[r0 + nz + z], Uc[r0 + 2 * nz + z]);
-        const f2 up = make_float2(Uc[r0 + nz + zp], Uc[r0 + 2 * nz + zp]);
+        const float* Uc = U + c * NRU * NZ;
+        const int r0 = (2 * t) * NZ;
+        mine[c] = make_float2(Uc[r0 + NZ + z], Uc[r0 + 2 * NZ + z]);
+        const f2 up = make_float2(Uc[r0 + NZ + zp], Uc[r0 + 2 * NZ + zp]);
         h[c][0] = make_float2(Uc[r0 + z], mine[c].x);
         h[c][1] = make_float2(Uc[r0 + zp], up.x);
         h[c][2] = mine[c];
@@ -1482,11 +1529,11 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
       f2 y[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        y[c] = p_add(own[c], Qab[pt + c * nz + zm]);
-        y[c].y += Qcd[pa + c * nz + z].x + Qcd[pa + c * nz + zm].y;
+        y[c] = p_add(own[c], Qab[pt + c * NZ + zm]);
+        y[c].y += Qcd[pa + c * NZ + z].x + Qcd[pa + c * NZ + zm].y;
       }
       float* ob = obase + pg;
-      const int r1 = (2 * t) * nz + z, r2 = r1 + nz;
+      const int r1 = (2 * t) * NZ + z, r2 = r1 + NZ;
       if (OUT == OUT_APPLY || OUT == OUT_APPLY_DOT) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -1553,7 +1600,7 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
       wait_stage(g);
       __syncthreads();
       if (abort_flag) break;
-      if (tid < 32 && g + kBulkSlots - 1 < G) issue(g + kBulkSlots - 1);
+      if (issuer && g + kBulkSlots - 1 < G) issue(g + kBulkSlots - 1);
       const float* S = stg + ((gbase + (unsigned)g) % kBulkSlots) * SS;
       const int pe = pe_next;
       pe_next += plane;
@@ -1586,8 +1633,8 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
           }
       }
       {
-        const float* K = S + oK + (2 * t) * nz + z;
-        const f2 kv = make_float2(K[0], K[nz]);
+        const float* K = S + oK + (2 * t) * NZ + z;
+        const f2 kv = make_float2(K[0], K[NZ]);
         const f2 A = p_mul(kv, a.kp[0]), Bdo = p_mul(kv, a.kp[1]), Bo = p_mul(kv, a.kp[2]);
         const f2 D1o = p_mul(kv, a.kp[3]), O1 = p_mul(kv, a.kp[4]);
         const f2 D2o = p_mul(kv, a.kp[5]), O2 = p_mul(kv, a.kp[6]), Gd = p_mul(kv, a.kp[7]);
@@ -1638,8 +1685,8 @@ stencil2b_kernel(StencilArgs<float, float, float, float> a) {
         u12[c] = raw[c];
         raw[c] = cur0[c];
         if (s > 0) {
-          Qab[pt + c * nz + z] = make_float2(tot[1].y + tot[3].x, tot[3].y);
-          Qcd[pt + c * nz + z] = make_float2(tot[0].x, tot[1].x);
+          Qab[pt + c * NZ + z] = make_float2(tot[1].y + tot[3].x, tot[3].y);
+          Qcd[pt + c * NZ + z] = make_float2(tot[0].x, tot[1].x);
         }
       }
       pg = pe;
@@ -1677,12 +1724,12 @@ __device__ __forceinline__ void had4s_inv(T (&v)[4]) {
 // carried lower plane transformed in y and z and the upper-plane
 // contributions half transformed (as in stencilp_kernel), arithmetic in FP64.
 // Thread (r, z) streams voxel (i, j0-1+r, z); row 0 is the y halo.  Stage
-// layout: U[3][R+1][nz] (TIn), KC[R][nz], B[3][R-1][nz] (double), ID[R-1][nz]
-// (float); Q[2][R][3 corners][3][nz] doubles.
+// layout: U[3][R+1][NZ] (TIn), KC[R][NZ], B[3][R-1][NZ] (double), ID[R-1][NZ]
+// (float); Q[2][R][3 corners][3][NZ] doubles.  NZ is the row pitch, as there.
 template <int NT, int OUT, int NZ, typename TIn>
 __global__ void __launch_bounds__(NT, 1)
 stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
-  static_assert(NZ > 0 && NZ % 4 == 0, "staged rows need a compile-time z extent, multiple of 4");
+  static_assert(NZ > 0 && NZ % 4 == 0 && NT % NZ == 0, "staged rows need a compile-time pitch, multiple of 4");
   constexpr int R = NT / NZ, NRU = R + 1, NRK = R, RB = R - 1;
   constexpr int bU = 0, bK = bU + 3 * NRU * NZ * (int)sizeof(TIn), bB = bK + NRK * NZ * 8,
                 bI = bB + 3 * RB * NZ * 8;
@@ -1694,11 +1741,11 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
   const CellDesc cd = a.cells[un.cell];
   if (a.stt && !a.stt[cd.id * kNumRhs + rhs].active) return;
   const int nx = cd.nx, ny = cd.ny;
-  constexpr int nz = NZ;
+  const int nz = cd.nz;
   const int tid = threadIdx.x;
-  const int r = tid / nz, z = tid - r * nz;
+  const int r = tid / NZ, z = tid - r * NZ;
   const int rows = un.rows;
-  const bool live = r <= rows;
+  const bool live = r <= rows && z < nz;
   const bool owner = live && r >= 1;
   const int zp = (z + 1 == nz) ? 0 : z + 1;
   const int zm = (z == 0) ? nz - 1 : z - 1;
@@ -1706,60 +1753,82 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
   const int jr = wrapy(un.j0 - 1 + r);
 
   unsigned char* stg = smem_raw;
-  double* Q = reinterpret_cast<double*>(stg + kBulkSlots * SSB);   // [2][R][3][3][nz]
+  double* Q = reinterpret_cast<double*>(stg + kBulkSlots * SSB);   // [2][R][3][3][NZ]
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(Q + 2 * QS);
   double* red = reinterpret_cast<double*>(bars + kBulkSlots);
   __shared__ int abort_flag;
-  const int qrow = r * 9 * nz, qup = (r > 0 ? r - 1 : 0) * 9 * nz;
+  const int qrow = r * 9 * NZ, qup = (r > 0 ? r - 1 : 0) * 9 * NZ;
 
   const long long st = a.ntot;
   const int plane = ny * nz;
   const int col = jr * nz + z;
   double* obase = a.out + (long long)rhs * 3 * st + cd.off;
 
+  // this thread's copy of every stage (bytes == 0: none)
   const char* src_base = nullptr;
   int plane_lag = 0, src_off = 0, dst_off = 0, bytes = 0, esz = 0;
   unsigned tx_total = 0;
-  if (tid < 32) {
-    int idx = 0;
-    auto seg = [&](const void* base, int es, int lag, int row0, int nrows, int dst) {
-      int done = 0;
-      while (done < nrows) {
-        const int r0 = wrapy(row0 + done);
-        const int n = min(nrows - done, ny - r0);
-        if (idx == tid) {
-          src_base = reinterpret_cast<const char*>(base);
-          esz = es;
-          plane_lag = lag;
-          src_off = r0 * nz;
-          dst_off = dst + done * nz * es;
-          bytes = n * nz * es;
+  const bool ids = (OUT == OUT_JACOBI || OUT == OUT_JACOBI_DOT) && !a.binv;
+  constexpr int esU = (int)sizeof(TIn);
+  if (nz == NZ) {
+    if (tid < 32) {
+      int idx = 0;
+      auto seg = [&](const void* base, int es, int lag, int row0, int nrows, int dst) {
+        int done = 0;
+        while (done < nrows) {
+          const int r0 = wrapy(row0 + done);
+          const int n = min(nrows - done, ny - r0);
+          if (idx == tid) {
+            src_base = reinterpret_cast<const char*>(base);
+            esz = es;
+            plane_lag = lag;
+            src_off = r0 * NZ;
+            dst_off = dst + done * NZ * es;
+            bytes = n * NZ * es;
+          }
+          tx_total += (unsigned)(n * NZ * es);
+          ++idx;
+          done += n;
         }
-        tx_total += (unsigned)(n * nz * es);
-        ++idx;
-        done += n;
+      };
+      for (int c = 0; c < 3; ++c)
+        seg(a.u + ((long long)rhs * 3 + c) * st + cd.off, esU, 1, un.j0 - 1, rows + 2, bU + c * NRU * NZ * esU);
+      seg(a.kc + cd.off, 8, 0, un.j0 - 1, rows + 1, bK);
+      if (OUT >= OUT_JACOBI) {
+        for (int c = 0; c < 3; ++c)
+          seg(a.b + ((long long)rhs * 3 + c) * st + cd.off, 8, -1, un.j0, rows, bB + c * RB * NZ * 8);
+        if (ids) seg(a.invd + cd.off, 4, -1, un.j0, rows, bI);
       }
-    };
-    for (int c = 0; c < 3; ++c)
-      seg(a.u + ((long long)rhs * 3 + c) * st + cd.off, (int)sizeof(TIn), 1, un.j0 - 1, rows + 2,
-          bU + c * NRU * nz * (int)sizeof(TIn));
-    seg(a.kc + cd.off, 8, 0, un.j0 - 1, rows + 1, bK);
-    if (OUT >= OUT_JACOBI) {
-      for (int c = 0; c < 3; ++c) seg(a.b + ((long long)rhs * 3 + c) * st + cd.off, 8, -1, un.j0, rows, bB + c * RB * nz * 8);
-      if (OUT != OUT_RESID && !a.binv) seg(a.invd + cd.off, 4, -1, un.j0, rows, bI);
     }
+  } else {
+    const int n[8] = {rows + 2, rows + 2, rows + 2, rows + 1, OUT >= OUT_JACOBI ? rows : 0,
+                      OUT >= OUT_JACOBI ? rows : 0, OUT >= OUT_JACOBI ? rows : 0, ids ? rows : 0};
+    int row = 0;
+    const int k8 = bulk_rows<8>((tid & 31) * (NT / 32) + (tid >> 5), n, row);
+    if (k8 >= 0) {
+      const int c = k8 < 3 ? k8 : k8 - 4;   // component of a u or b row
+      src_base = k8 < 3    ? reinterpret_cast<const char*>(a.u + ((long long)rhs * 3 + c) * st + cd.off)
+                 : k8 == 3 ? reinterpret_cast<const char*>(a.kc + cd.off)
+                 : k8 < 7  ? reinterpret_cast<const char*>(a.b + ((long long)rhs * 3 + c) * st + cd.off)
+                           : reinterpret_cast<const char*>(a.invd + cd.off);
+      esz = k8 < 3 ? esU : k8 < 7 ? 8 : 4;
+      plane_lag = k8 < 3 ? 1 : k8 == 3 ? 0 : -1;
+      src_off = wrapy(un.j0 - (k8 < 4 ? 1 : 0) + row) * nz;
+      dst_off = k8 < 3 ? bU + (c * NRU + row) * NZ * esU : k8 == 3 ? bK + row * NZ * 8
+                : k8 < 7 ? bB + (c * RB + row) * NZ * 8 : bI + row * NZ * 4;
+      bytes = nz * esz;
+    }
+    tx_total = (unsigned)nz * (unsigned)(esU * (n[0] + n[1] + n[2]) + 8 * (n[3] + n[4] + n[5] + n[6]) + 4 * n[7]);
   }
+  const bool issuer = tid == 0 || bytes > 0;
   int pl_next = ((un.i0 - 2 + plane_lag) % nx + nx) % nx;
   int issued = 0;
   auto issue = [&](int g) {
     issued = g + 1;
     const int slot = g % kBulkSlots;
     const unsigned bar = smem_addr(bars + slot);
-    if (tid == 0) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_expect_tx(bar, tx_total);
-    }
-    __syncwarp();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (tid == 0) mbar_expect_tx(bar, tx_total);
     if (bytes > 0)
       bulk_g2s(smem_addr(stg + slot * SSB + dst_off), src_base + (long long)esz * ((long long)pl_next * plane + src_off),
                (unsigned)bytes, bar);
@@ -1772,7 +1841,7 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  if (tid < 32)
+  if (issuer)
     for (int g = 0; g < kBulkSlots && g < G; ++g) issue(g);
   int waited = 0;   // stages 0 .. waited-1 completed for this thread (the exit drain starts there)
   auto wait_stage = [&](int g) {
@@ -1792,24 +1861,24 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
     const TIn* U = reinterpret_cast<const TIn*>(S + bU);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const TIn* Uc = U + c * NRU * nz + r * nz;
+      const TIn* Uc = U + c * NRU * NZ + r * NZ;
       mine[c] = (double)Uc[z];
       h[c][0] = mine[c];
       h[c][1] = (double)Uc[zp];
-      h[c][2] = (double)Uc[nz + z];
-      h[c][3] = (double)Uc[nz + zp];
+      h[c][2] = (double)Uc[NZ + z];
+      h[c][3] = (double)Uc[NZ + zp];
       had4s_fwd(h[c]);
     }
   };
   auto gather = [&](int buf, const unsigned char* S) {
     const double* Qg = Q + buf * QS;
     double* ob = obase + pg + col;
-    const int rb = (r - 1) * nz + z;   // owned row in the b / invd arrays
+    const int rb = (r - 1) * NZ + z;   // owned row in the b / invd arrays
     const double* Bs = reinterpret_cast<const double*>(S + bB);
     double y[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
-      y[c] = own[c] + Qg[qrow + (0 * 3 + c) * nz + zm] + Qg[qup + (1 * 3 + c) * nz + z] + Qg[qup + (2 * 3 + c) * nz + zm];
+      y[c] = own[c] + Qg[qrow + (0 * 3 + c) * NZ + zm] + Qg[qup + (1 * 3 + c) * NZ + z] + Qg[qup + (2 * 3 + c) * NZ + zm];
     if (OUT == OUT_APPLY || OUT == OUT_APPLY_DOT) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -1818,12 +1887,12 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
       }
     } else if (OUT == OUT_RESID) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) ob[c * st] = Bs[c * RB * nz + rb] - y[c];
+      for (int c = 0; c < 3; ++c) ob[c * st] = Bs[c * RB * NZ + rb] - y[c];
     } else {
       const float* Is = reinterpret_cast<const float*>(S + bI);
       double dv[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) dv[c] = Bs[c * RB * nz + rb] - y[c];
+      for (int c = 0; c < 3; ++c) dv[c] = Bs[c * RB * NZ + rb] - y[c];
       if (a.binv) {   // node-block sweep: the node's block inverse, read where the gather needs it
         jacobi_dir<double>(a.binv, cd.off + pg + col, 0.0, dv);
 #pragma unroll
@@ -1837,7 +1906,7 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
       for (int c = 0; c < 3; ++c) {
         const double xv = unode[c] + dv[c];
         ob[c * st] = xv;
-        if (OUT == OUT_JACOBI_DOT) acc += xv * Bs[c * RB * nz + rb];
+        if (OUT == OUT_JACOBI_DOT) acc += xv * Bs[c * RB * NZ + rb];
       }
     }
   };
@@ -1860,7 +1929,7 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
     wait_stage(g);
     __syncthreads();
     if (abort_flag) break;
-    if (tid < 32 && g + kBulkSlots - 1 < G) issue(g + kBulkSlots - 1);
+    if (issuer && g + kBulkSlots - 1 < G) issue(g + kBulkSlots - 1);
     const unsigned char* S = stg + (g % kBulkSlots) * SSB;
     const int pe = pe_next;
     pe_next += plane;
@@ -1881,7 +1950,7 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
           prv[c][q] = cur[c][q];
         }
     }
-    had_block(w, a.k, reinterpret_cast<const double*>(S + bK)[r * nz + z]);
+    had_block(w, a.k, reinterpret_cast<const double*>(S + bK)[r * NZ + z]);
     double* Qb = Q + (s & 1) * QS;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -1898,9 +1967,9 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
       unode[c] = rawn[c];
       rawn[c] = cur0[c];
       if (s > 0) {
-        Qb[qrow + (0 * 3 + c) * nz + z] = tot[1];   // node (jr, z+1)
-        Qb[qrow + (1 * 3 + c) * nz + z] = tot[2];   // node (jr+1, z)
-        Qb[qrow + (2 * 3 + c) * nz + z] = tot[3];   // node (jr+1, z+1)
+        Qb[qrow + (0 * 3 + c) * NZ + z] = tot[1];   // node (jr, z+1)
+        Qb[qrow + (1 * 3 + c) * NZ + z] = tot[2];   // node (jr+1, z)
+        Qb[qrow + (2 * 3 + c) * NZ + z] = tot[3];   // node (jr+1, z+1)
       }
     }
     pg = pe;

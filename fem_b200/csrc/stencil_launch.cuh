@@ -93,8 +93,8 @@ void stencil(femh_handle* H, Level& L, bool smooth_only, const TIn* in, TOut* ou
   if (!std::is_same<T, float>::value) {   // packed-FP32 kernels: FP64 twin with the same units
     if (variant == 3) variant = 1;
     if (variant == 4 || variant == 5 || variant == 7) variant = 2;
-  } else if (variant == 6) {   // the staged FP64 kernel's FP32 twin has the same units
-    variant = 1;
+  } else if (variant == 6) {   // the staged FP64 kernel's FP32 twin takes the same units
+    variant = 2;
   }
   if (variant == 6) {   // bulk-copy staging: FP64 output / rhs / coefficients, aligned rows
     const bool ok = std::is_same<TOut, double>::value && std::is_same<TB, double>::value &&
@@ -102,7 +102,7 @@ void stencil(femh_handle* H, Level& L, bool smooth_only, const TIn* in, TOut* ou
                     (std::is_same<TIn, double>::value || std::is_same<TIn, float>::value);
     auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
     if (!(ok && L.bulk_ok64 && al(in) && al(out) && al(kc) && al(L.invd) && (!b || al(b)) && L.ntot % 4 == 0))
-      variant = 1;
+      variant = 2;
   }
   bool persistent = false;
   if (variant == 7) {   // the staged kernel as persistent CTAs over the list's CTA table
@@ -173,31 +173,36 @@ void stencil(femh_handle* H, Level& L, bool smooth_only, const TIn* in, TOut* ou
                   std::is_same<TB, double>::value && std::is_same<TC, double>::value &&
                   (std::is_same<TIn, double>::value || std::is_same<TIn, float>::value)) {
       if (variant == 6) {
-        const size_t sm6 = stencil1b_smem_bytes(lnt, nz_spec, (int)sizeof(TIn));
-        switch (nz_spec) {
-          case 16: stencil_go6<512, OUT, 16>(H, grid, sm6, a); return;
-          case 24: stencil_go6<480, OUT, 24>(H, grid, sm6, a); return;
-          case 32: stencil_go6<512, OUT, 32>(H, grid, sm6, a); return;
-          case 48: stencil_go6<480, OUT, 48>(H, grid, sm6, a); return;
-          case 64: stencil_go6<512, OUT, 64>(H, grid, sm6, a); return;
-          case 128: stencil_go6<512, OUT, 128>(H, grid, sm6, a); return;
-          case 256: stencil_go6<512, OUT, 256>(H, grid, sm6, a); return;
+        const int c = stage_class(nz_spec > 0 ? nz_spec : maxnz);
+        const size_t sm6 = stencil1b_smem_bytes(stage_nt64(c), c, (int)sizeof(TIn));
+        switch (c) {
+          case 16: stencil_go6<stage_nt64(16), OUT, 16>(H, grid, sm6, a); return;
+          case 24: stencil_go6<stage_nt64(24), OUT, 24>(H, grid, sm6, a); return;
+          case 32: stencil_go6<stage_nt64(32), OUT, 32>(H, grid, sm6, a); return;
+          case 48: stencil_go6<stage_nt64(48), OUT, 48>(H, grid, sm6, a); return;
+          case 64: stencil_go6<stage_nt64(64), OUT, 64>(H, grid, sm6, a); return;
+          case 96: stencil_go6<stage_nt64(96), OUT, 96>(H, grid, sm6, a); return;
+          case 128: stencil_go6<stage_nt64(128), OUT, 128>(H, grid, sm6, a); return;
+          case 192: stencil_go6<stage_nt64(192), OUT, 192>(H, grid, sm6, a); return;
+          case 256: stencil_go6<stage_nt64(256), OUT, 256>(H, grid, sm6, a); return;
           default: throw FemhError{FEMH_E_ARG, "staged FP64 stencil on an ineligible level"};
         }
       }
     }
     if constexpr (std::is_same<TIn, float>::value && std::is_same<TOut, float>::value &&
                   std::is_same<TB, float>::value && std::is_same<TC, float>::value) {
-      if (variant == 5) {   // eligible levels have a compile-time z extent and 384-thread tiles
-        const int nt = variant_nt(lnt, maxnz, 5);
-        const size_t sm5 = stencil2b_smem_bytes(nt, nz_spec);
-        switch (nz_spec) {
-          case 16: stencil_go5<384, OUT, 16>(H, grid, sm5, a); return;
-          case 24: stencil_go5<384, OUT, 24>(H, grid, sm5, a); return;
-          case 32: stencil_go5<384, OUT, 32>(H, grid, sm5, a); return;
-          case 48: stencil_go5<384, OUT, 48>(H, grid, sm5, a); return;
-          case 64: stencil_go5<384, OUT, 64>(H, grid, sm5, a); return;
-          case 128: stencil_go5<384, OUT, 128>(H, grid, sm5, a); return;
+      if (variant == 5) {
+        const int c = stage_class(nz_spec > 0 ? nz_spec : maxnz);
+        const size_t sm5 = stencil2b_smem_bytes(kStageNT32, c);
+        switch (c) {
+          case 16: stencil_go5<kStageNT32, OUT, 16>(H, grid, sm5, a); return;
+          case 24: stencil_go5<kStageNT32, OUT, 24>(H, grid, sm5, a); return;
+          case 32: stencil_go5<kStageNT32, OUT, 32>(H, grid, sm5, a); return;
+          case 48: stencil_go5<kStageNT32, OUT, 48>(H, grid, sm5, a); return;
+          case 64: stencil_go5<kStageNT32, OUT, 64>(H, grid, sm5, a); return;
+          case 96: stencil_go5<kStageNT32, OUT, 96>(H, grid, sm5, a); return;
+          case 128: stencil_go5<kStageNT32, OUT, 128>(H, grid, sm5, a); return;
+          case 192: stencil_go5<kStageNT32, OUT, 192>(H, grid, sm5, a); return;
           default: throw FemhError{FEMH_E_ARG, "bulk-copy stencil on an ineligible level"};
         }
       }
