@@ -697,7 +697,11 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
   H->d_part_b = ar.arr<double>(H->part_g_slots * H->bsub * kNumRhs);
   H->d_bcg = ar.arr<BlockCG>(nc);
   H->d_part_z = ar.arr<double>(std::max(L0.all.nu.size(), L0.all.su.size()) * kNumRhs);
-  H->d_part_e = ar.arr<double>(L0.all.nu.size() * 22);   // 21 pair energies + sum of rho per slot
+  // energy kernels (three 128-thread CTAs per SM, 64 voxels a pass): at least
+  // eight CTAs per SM, down to one pass each (a 16^3 cell ran on 2 CTAs)
+  H->bsub_e = 1;
+  while (H->bsub_e < 32 && (long long)H->part_g_slots * H->bsub_e < 8 * nsm) H->bsub_e *= 2;
+  H->d_part_e = ar.arr<double>(L0.all.nu.size() * H->bsub_e * 22);   // 21 pair energies + sum of rho per sub-slot
   H->d_C = ar.arr<double>(nc * 36);
   H->d_W = ar.arr<double>(nc * 21);
   H->d_nrm = ar.arr<double>(nc * kNumRhs);
@@ -1727,32 +1731,43 @@ void solve_all(femh_handle* H, std::vector<femh_solve_info>& infos) {
   }
 }
 
-// Energy pairs of the resident fields: C^H with the element matrix's Hadamard
-// factors k = H->hk; other factors give other bilinear forms on the same fields.
-void energy_C(femh_handle* H, std::vector<double>& C, std::vector<double>& dens, const HadK* k = nullptr) {
+// Arguments of the energy kernels on the resident fields.
+EnergyArgs energy_args(femh_handle* H, const HadK& k) {
   Level& L0 = H->levels[0];
-  cudaStream_t s = H->stream;
   EnergyArgs a{};
   a.cells = L0.d_cells;
   a.units = L0.all.d_nu;
   a.chi = H->x64;
   a.kc64 = H->kc64;
   a.rho = H->rho_used;
-  a.ec = H->d_ec;
+  a.W = H->d_W;
   a.part = H->d_part_e;
   a.ntot = L0.ntot;
-  a.k = k ? *k : H->hk;
+  a.nsub = H->bsub_e;
+  a.m = energy_modes(k, H->ec);
   a.law = make_law(H->cfg);
-  {
-    Prof prof_(H, "k_energy", 0.0);
-    k_energy<EN_C><<<(unsigned)L0.all.nu.size(), 128, 0, s>>>(a);
-    LAUNCH_CHECK(H);
-  }
+  return a;
+}
+template <int MODE>
+void energy_launch(femh_handle* H, const EnergyArgs& a) {
+  const double per = MODE == EN_DCDRHO ? 328.0 : 168.0;   // bytes per voxel
+  Prof prof_(H, MODE == EN_C ? "k_energy_C" : (MODE == EN_GRAD ? "k_energy_grad" : "k_energy_table"),
+             per * (double)H->nvox);
+  k_energy<MODE><<<(unsigned)(H->levels[0].all.nu.size() * a.nsub), 128, 0, H->stream>>>(a);
+  LAUNCH_CHECK(H);
+}
+
+// Energy pairs of the resident fields: C^H with the element matrix's Hadamard
+// factors k = H->hk; other factors give other bilinear forms on the same fields.
+void energy_C(femh_handle* H, std::vector<double>& C, std::vector<double>& dens, const HadK* k = nullptr) {
+  Level& L0 = H->levels[0];
+  cudaStream_t s = H->stream;
+  energy_launch<EN_C>(H, energy_args(H, k ? *k : H->hk));
   double* d_dens = H->d_nrm;
   {
     Prof prof_(H, "k_energy_fin", 0.0);
-    k_energy_fin<<<cdiv((long long)H->ncells * 22, 128), 128, 0, s>>>(L0.d_cells, L0.d_nu_sb, L0.d_nu_se,
-                                                                   H->d_part_e, H->d_C, d_dens, H->ncells);
+    k_energy_fin<<<cdiv((long long)H->ncells * 22 * 32, 128), 128, 0, s>>>(
+        L0.d_cells, L0.d_nu_sb, L0.d_nu_se, H->d_part_e, H->d_C, d_dens, H->ncells, H->bsub_e);
     LAUNCH_CHECK(H);
   }
   C.assign(H->ncells * 36, 0.0);
@@ -2005,23 +2020,9 @@ femh_status femh_homogenize_batch(femh_handle* H, int ncell, const femh_cell* ce
             W[ci * 21 + t++] = (I == J) ? dLdC[ci * 36 + I * 6 + I] : dLdC[ci * 36 + I * 6 + J] + dLdC[ci * 36 + J * 6 + I];
       }
       CK(cudaMemcpyAsync(H->d_W, W.data(), sizeof(double) * W.size(), cudaMemcpyHostToDevice, H->stream));
-      EnergyArgs a{};
-      a.cells = L0.d_cells;
-      a.units = L0.all.d_nu;
-      a.chi = H->x64;
-      a.kc64 = H->kc64;
-      a.rho = H->rho_used;
-      a.ec = H->d_ec;
-      a.W = H->d_W;
+      EnergyArgs a = energy_args(H, H->hk);
       a.out = grad_target(H, dLdrho, 0);
-      a.ntot = L0.ntot;
-      a.k = H->hk;
-      a.law = make_law(H->cfg);
-      {
-        Prof prof_(H, "k_energy", 0.0);
-        k_energy<EN_GRAD><<<(unsigned)L0.all.nu.size(), 128, 0, H->stream>>>(a);
-        LAUNCH_CHECK(H);
-      }
+      energy_launch<EN_GRAD>(H, a);
       to_host_or_dev(H, dLdrho, a.out, H->nvox, 0);
     }
   });
@@ -2040,23 +2041,9 @@ femh_status femh_homogenize_grad(femh_handle* H, const double dLdC[36], double* 
     for (int I = 0; I < 6; ++I)
       for (int J = 0; J <= I; ++J) W[t++] = (I == J) ? dLdC[I * 6 + I] : dLdC[I * 6 + J] + dLdC[J * 6 + I];
     CK(cudaMemcpyAsync(H->d_W, W, sizeof W, cudaMemcpyHostToDevice, H->stream));
-    EnergyArgs a{};
-    a.cells = L0.d_cells;
-    a.units = L0.all.d_nu;
-    a.chi = H->x64;
-    a.kc64 = H->kc64;
-    a.rho = H->rho_used;
-    a.ec = H->d_ec;
-    a.W = H->d_W;
+    EnergyArgs a = energy_args(H, H->hk);
     a.out = grad_target(H, dLdrho, out_on_device);
-    a.ntot = L0.ntot;
-    a.k = H->hk;
-    a.law = make_law(H->cfg);
-    {
-      Prof prof_(H, "k_energy", 0.0);
-      k_energy<EN_GRAD><<<(unsigned)L0.all.nu.size(), 128, 0, H->stream>>>(a);
-      LAUNCH_CHECK(H);
-    }
+    energy_launch<EN_GRAD>(H, a);
     if (!out_on_device) to_host_or_dev(H, dLdrho, a.out, H->nvox, 0);
   });
 }
@@ -2107,26 +2094,12 @@ femh_status femh_field_gradient(femh_handle* H, const double dLdC[36], double dL
     for (int I = 0; I < 6; ++I)
       for (int J = 0; J <= I; ++J) W[t++] = (I == J) ? dLdC[I * 6 + I] : dLdC[I * 6 + J] + dLdC[J * 6 + I];
     CK(cudaMemcpyAsync(H->d_W, W, sizeof W, cudaMemcpyHostToDevice, H->stream));
-    EnergyArgs a{};
-    a.cells = L0.d_cells;
-    a.units = L0.all.d_nu;
-    a.chi = H->x64;
-    a.kc64 = H->kc64;
-    a.rho = H->rho_used;
-    a.ec = H->d_ec;
-    a.W = H->d_W;
+    EnergyArgs a = energy_args(H, H->hk);
     // the voxel gradient and then the parameter sums, in the dead CG buffer q
     // when they fit (18 x nvox FP64 or FP32 values), else in the staging buffer
     const size_t qd = (size_t)18 * nv * (H->cfg.precision == FEMH_MIXED ? 4 : 8) / sizeof(double);
     a.out = ((size_t)nv + nparam <= qd) ? grad_target(H, nullptr, 0) : stage(H, (size_t)nv + nparam);
-    a.ntot = L0.ntot;
-    a.k = H->hk;
-    a.law = make_law(H->cfg);
-    {
-      Prof prof_(H, "k_energy", 0.0);
-      k_energy<EN_GRAD><<<(unsigned)L0.all.nu.size(), 128, 0, H->stream>>>(a);
-      LAUNCH_CHECK(H);
-    }
+    energy_launch<EN_GRAD>(H, a);
     double* pg = a.out + nv;
     {
       Prof prof_(H, "k_param_sum", 0.0);
@@ -2168,22 +2141,9 @@ femh_status femh_dCdrho(femh_handle* H, double* out, int out_on_device) {
     if (!out) throw FemhError{FEMH_E_ARG, "out must not be NULL"};
     CK(cudaSetDevice(H->device));
     Level& L0 = H->levels[0];
-    EnergyArgs a{};
-    a.cells = L0.d_cells;
-    a.units = L0.all.d_nu;
-    a.chi = H->x64;
-    a.kc64 = H->kc64;
-    a.rho = H->rho_used;
-    a.ec = H->d_ec;
+    EnergyArgs a = energy_args(H, H->hk);
     a.out = out_on_device ? out : stage(H, 21 * (size_t)H->nvox);
-    a.ntot = L0.ntot;
-    a.k = H->hk;
-    a.law = make_law(H->cfg);
-    {
-      Prof prof_(H, "k_energy", 0.0);
-      k_energy<EN_DCDRHO><<<(unsigned)L0.all.nu.size(), 128, 0, H->stream>>>(a);
-      LAUNCH_CHECK(H);
-    }
+    energy_launch<EN_DCDRHO>(H, a);
     if (!out_on_device) to_host_or_dev(H, out, a.out, 21 * H->nvox, 0);
   });
 }

@@ -21,13 +21,17 @@ struct MatLaw {
   double E_s, E_min, penal, bin_hi, bin_lo, rho_min, rho_max;
 };
 
+// SIMP's usual exponent 3 needs no pow (whose ~100 instructions are half of what
+// the density gradient does per voxel besides the field sums).
 __host__ __device__ inline double law_coef(const MatLaw& m, double rho) {
-  if (m.interp == INTERP_SIMP) return m.E_min + pow(rho, m.penal) * (m.E_s - m.E_min);
+  if (m.interp == INTERP_SIMP)
+    return m.E_min + (m.penal == 3.0 ? rho * rho * rho : pow(rho, m.penal)) * (m.E_s - m.E_min);
   if (m.interp == INTERP_RAMP3) return m.E_s * rho / (3.0 - 2.0 * rho);
   return rho >= 0.5 ? m.bin_hi : m.bin_lo;
 }
 __host__ __device__ inline double law_dcoef(const MatLaw& m, double rho) {
-  if (m.interp == INTERP_SIMP) return m.penal * pow(rho, m.penal - 1.0) * (m.E_s - m.E_min);
+  if (m.interp == INTERP_SIMP)
+    return m.penal * (m.penal == 3.0 ? rho * rho : pow(rho, m.penal - 1.0)) * (m.E_s - m.E_min);
   if (m.interp == INTERP_RAMP3) {
     const double d = 3.0 - 2.0 * rho;
     return m.E_s * 3.0 / (d * d);
@@ -1191,111 +1195,228 @@ __global__ void k_coarse_solve(const CellDesc* cells, const int* list, const dou
 }
 
 // ------------------------------------------------------- energy kernels ---
-// Per voxel: u^I = ue0^I(h) + chi^I (6 load cases), uhat = T u, w = Kh uhat;
-// s_IJ = uhat^I . w^J = u^I . K0(1) u^J.  Modes:
-//   C partials:   sum_e kc_e s_IJ       (-> C^H = sum / (|Y|))     [slot][21]
+// Per voxel: u^I = ue0^I(h) + chi^I (6 load cases) and the 21 pairs
+// s_IJ = u^I . K0(1) u^J.  Modes:
+//   C partials:   sum_e kc_e s_IJ       (-> C^H = sum / (|Y|))     [sub-slot][22]
 //   dC/drho:      out[t][e] = c'(rho_e) h s_t / |Y|
 //   dL/drho:      out[e] = c'(rho_e) h sum_t W_t s_t / |Y|
 enum EnergyMode : int { EN_C = 0, EN_DCDRHO = 1, EN_GRAD = 2 };
+
+// K0 in the 18 strain modes of the voxel, in which it is diagonal:
+// s_IJ = sum_k w_k phi_k^I phi_k^J.  The modes are the Hadamard coefficients
+// that carry energy, combined to the eigenvectors of Kh's 3x3 and 2x2 blocks
+// (a block d I + o J has the sum with weight (d + 2 o) / 3 and two differences
+// with (d - o) / 2 and (d - o) / 6, or (d +- o) / 2 for a pair; the shear pairs
+// have the sum only).  The macro strains reach the first six modes.
+struct EnergyModes {
+  double nsum, nd1, nd2, shear, msum, md1, md2, psum, pdif, cube;   // weights
+  double m0[kNumRhs][6];   // unit macro strains (h = 1): normal sum, differences 1 and 2, shear xz, yz, xy
+};
+inline EnergyModes energy_modes(const HadK& k, const ElemConst& ec) {
+  EnergyModes m{};
+  m.nsum = (k.Bd + 2 * k.Bo) / 3;
+  m.nd1 = (k.Bd - k.Bo) / 2;
+  m.nd2 = (k.Bd - k.Bo) / 6;
+  m.shear = k.A;
+  m.msum = (k.D1 + 2 * k.O1) / 3;
+  m.md1 = (k.D1 - k.O1) / 2;
+  m.md2 = (k.D1 - k.O1) / 6;
+  m.psum = (k.D2 + k.O2) / 2;
+  m.pdif = (k.D2 - k.O2) / 2;
+  m.cube = k.G;
+  for (int I = 0; I < kNumRhs; ++I) {
+    const auto& u = ec.uhat0[I];
+    const double n0 = u[0][4], n1 = u[1][2], n2 = u[2][1];
+    m.m0[I][0] = n0 + n1 + n2;
+    m.m0[I][1] = n0 - n1;
+    m.m0[I][2] = n0 + n1 - 2 * n2;
+    m.m0[I][3] = u[0][1] + u[2][4];
+    m.m0[I][4] = u[1][1] + u[2][2];
+    m.m0[I][5] = u[0][2] + u[1][4];
+  }
+  return m;
+}
+
 struct EnergyArgs {
   const CellDesc* cells;
   const NodeUnit* units;
   const double* chi;      // [6][3][ntot] FP64
   const double* kc64;     // c_e * h
   const double* rho;      // rho actually used (clamped)
-  const ElemConst* ec;
   const double* W;        // [cell][21] symmetric weights for EN_GRAD
-  double* part;           // EN_C: [slot][21]
+  double* part;           // EN_C: [sub-slot][22]
   double* out;            // EN_DCDRHO: [21][ntot]; EN_GRAD: [ntot]
   long long ntot;
-  HadK k;
+  int nsub;               // CTAs per node unit
+  EnergyModes m;
   MatLaw law;
 };
 
-template <int MODE>
-__global__ void __launch_bounds__(128) k_energy(EnergyArgs a) {
-  const NodeUnit u = a.units[blockIdx.x];
-  const CellDesc cd = a.cells[u.cell];
-  const double vol = (double)cd.nx * cd.ny * cd.nz * cd.h * cd.h * cd.h;
-  double acc[22];
+// 18 modes of one load case of a voxel: chi = its x component (components ntot
+// apart), nd = the 8 corner nodes, m0 = the macro strain's modes.
+__device__ __forceinline__ void energy_phi(const double* __restrict__ chi, long long ntot, const unsigned (&nd)[8],
+                                           double h, const double (&m0)[6], double (&f)[18]) {
+  double w[3][8];
 #pragma unroll
-  for (int t = 0; t < 22; ++t) acc[t] = 0.0;
-  for (long long e = u.begin + threadIdx.x; e < u.end; e += blockDim.x) {
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int a8 = 0; a8 < 8; ++a8) w[c][a8] = chi[c * ntot + nd[a8]];
+    fwht8_fwd(w[c]);
+  }
+  f[0] = w[0][4] + w[1][2] + w[2][1] + h * m0[0];
+  f[1] = w[0][4] - w[1][2] + h * m0[1];
+  f[2] = w[0][4] + w[1][2] - 2.0 * w[2][1] + h * m0[2];
+  f[3] = w[0][1] + w[2][4] + h * m0[3];
+  f[4] = w[1][1] + w[2][2] + h * m0[4];
+  f[5] = w[0][2] + w[1][4] + h * m0[5];
+  f[6] = w[0][3] + w[1][5] + w[2][6];
+  f[7] = w[0][3] - w[1][5];
+  f[8] = w[0][3] + w[1][5] - 2.0 * w[2][6];
+  f[9] = w[1][3] + w[0][5];
+  f[10] = w[1][3] - w[0][5];
+  f[11] = w[2][3] + w[0][6];
+  f[12] = w[2][3] - w[0][6];
+  f[13] = w[2][5] + w[1][6];
+  f[14] = w[2][5] - w[1][6];
+  f[15] = w[0][7];
+  f[16] = w[1][7];
+  f[17] = w[2][7];
+}
+
+// Two threads per voxel: a warp's lower half holds the modes of load cases 0-2
+// of 16 voxels, its upper half those of cases 3-5 of the same voxels; mode by
+// mode they exchange their three values and each adds up 12 of the pairs
+// (its own 6; three across; the three pairs (i, i + 3) in both halves).
+// One thread per voxel needed the 144 coefficients of all cases at once and
+// spilled; this takes 108 registers of modes and one pass over the fields.
+// Bound by its instruction mix at 12 warps per SM: per 16 voxels ~525 FP64
+// operations, 72 loads and 108 shuffles a lane, and prefetching the next
+// fields changes nothing.  96^3: 206 -> 137 us (table) and 140 (gradient),
+// 0.35 of measured HBM for the table; 24^3 both 46 -> 14 us (more CTAs).
+// Pair p of half h is entry kEnergyPair[h][p] of the lower triangle.
+__device__ constexpr signed char kEnergyPair[2][12] = {
+    {0, 1, 3, 2, 4, 5, /* (0,4) (0,5) (1,5) */ 10, 15, 16, /* (0,3) (1,4) (2,5) */ 6, 11, 17},
+    {9, 13, 18, 14, 19, 20, /* (3,1) (3,2) (4,2) */ 7, 8, 12, /* as in half 0 */ 6, 11, 17}};
+
+template <int MODE>
+__global__ void __launch_bounds__(128, 3) k_energy(EnergyArgs a) {
+  const SubUnit su = sub_unit(a.units, a.nsub);
+  const CellDesc cd = a.cells[su.u.cell];
+  const double vol = (double)cd.nx * cd.ny * cd.nz * cd.h * cd.h * cd.h;
+  const int half = (threadIdx.x >> 4) & 1;
+  const int lane16 = threadIdx.x & 15, warp = threadIdx.x >> 5;
+  const double* chi = a.chi + (long long)half * 9 * a.ntot + cd.off;
+  double acc[12], rsum = 0.0;
+#pragma unroll
+  for (int p = 0; p < 12; ++p) acc[p] = 0.0;
+  for (long long e0 = su.begin + warp * 16; e0 < su.end; e0 += 64) {
+    const bool in = e0 + lane16 < su.end;
+    const long long e = in ? e0 + lane16 : su.end - 1;   // idle lanes repeat the last voxel, unweighted
     int i, j, k;
     node_ijk(e, cd.ny, cd.nz, i, j, k);
-    long long nd[8];
+    unsigned nd[8];
 #pragma unroll
     for (int a8 = 0; a8 < 8; ++a8)
-      nd[a8] = cd.off + lin(wrap(i + ((a8 >> 2) & 1), cd.nx), wrap(j + ((a8 >> 1) & 1), cd.ny),
-                            wrap(k + (a8 & 1), cd.nz), cd.ny, cd.nz);
-    double uh[kNumRhs][3][8];
+      nd[a8] = (unsigned)lin(wrap(i + ((a8 >> 2) & 1), cd.nx), wrap(j + ((a8 >> 1) & 1), cd.ny),
+                             wrap(k + (a8 & 1), cd.nz), cd.ny, cd.nz);
+    double f[3][18];
 #pragma unroll
-    for (int I = 0; I < kNumRhs; ++I)
+    for (int q = 0; q < 3; ++q) {
+      double m0[6];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
+      for (int t = 0; t < 6; ++t) m0[t] = half ? a.m.m0[q + 3][t] : a.m.m0[q][t];
+      energy_phi(chi + (long long)q * 3 * a.ntot, a.ntot, nd, cd.h, m0, f[q]);
+    }
+    double s[12];
 #pragma unroll
-        for (int a8 = 0; a8 < 8; ++a8) uh[I][c][a8] = a.chi[((long long)I * 3 + c) * a.ntot + nd[a8]];
-        fwht8_fwd(uh[I][c]);
+    for (int p = 0; p < 12; ++p) s[p] = 0.0;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) uh[I][c][kk] += cd.h * a.ec->uhat0[I][c][kk];
-      }
-    double s[21];
-#pragma unroll
-    for (int J = 0; J < kNumRhs; ++J) {
-      double w[3][8];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) w[c][kk] = uh[J][c][kk];
-      had_block(w, a.k, 1.0);
-#pragma unroll
-      for (int I = J; I < kNumRhs; ++I) {
-        double d = 0.0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int kk = 1; kk < 8; ++kk) d += uh[I][c][kk] * w[c][kk];
-        s[I * (I + 1) / 2 + J] = d;   // u^I.K0 u^J = (T u^I).Kh (T u^J)
-      }
+    for (int t = 0; t < 18; ++t) {
+      const double w = t == 0 ? a.m.nsum : t == 1 ? a.m.nd1 : t == 2 ? a.m.nd2 : t < 6 ? a.m.shear : t == 6 ? a.m.msum
+                       : t == 7 ? a.m.md1 : t == 8 ? a.m.md2 : t < 15 ? (t % 2 ? a.m.psum : a.m.pdif) : a.m.cube;
+      const double x0 = f[0][t], x1 = f[1][t], x2 = f[2][t];
+      const double y0 = __shfl_xor_sync(0xffffffffu, x0, 16), y1 = __shfl_xor_sync(0xffffffffu, x1, 16),
+                   y2 = __shfl_xor_sync(0xffffffffu, x2, 16);
+      const double w0 = w * x0, w1 = w * x1, w2 = w * x2;
+      s[0] += w0 * x0;
+      s[1] += w0 * x1;
+      s[2] += w0 * x2;
+      s[3] += w1 * x1;
+      s[4] += w1 * x2;
+      s[5] += w2 * x2;
+      s[6] += w0 * y1;
+      s[7] += w0 * y2;
+      s[8] += w1 * y2;
+      s[9] += w0 * y0;
+      s[10] += w1 * y1;
+      s[11] += w2 * y2;
     }
     if (MODE == EN_C) {
-      const double ke = a.kc64[cd.off + e];
+      const double ke = in ? a.kc64[cd.off + e] : 0.0;
 #pragma unroll
-      for (int t = 0; t < 21; ++t) acc[t] += ke * s[t];
-      acc[21] += a.rho[cd.off + e];
+      for (int p = 0; p < 12; ++p) acc[p] += ke * s[p];
+      if (in) rsum += a.rho[cd.off + e];
     } else {
       const double dc = law_dcoef(a.law, a.rho[cd.off + e]) * cd.h / vol;
       if (MODE == EN_DCDRHO) {
+        if (in) {
 #pragma unroll
-        for (int t = 0; t < 21; ++t) a.out[(long long)t * a.ntot + cd.off + e] = dc * s[t];
+          for (int p = 0; p < 12; ++p)
+            if (p < 9 || half == 0) a.out[(long long)kEnergyPair[half][p] * a.ntot + cd.off + e] = dc * s[p];
+        }
       } else {
         double g = 0.0;
 #pragma unroll
-        for (int t = 0; t < 21; ++t) g += a.W[cd.id * 21 + t] * s[t];
-        a.out[cd.off + e] = dc * g;
+        for (int p = 0; p < 12; ++p)
+          if (p < 9 || half == 0) g += a.W[cd.id * 21 + kEnergyPair[half][p]] * s[p];
+        g += __shfl_xor_sync(0xffffffffu, g, 16);
+        if (in && half == 0) a.out[cd.off + e] = dc * g;
       }
     }
   }
-  if (MODE == EN_C) {
-    __shared__ double red[32 * 22];
-    block_reduce<22>(acc, red);
-    if (threadIdx.x == 0)
+  if (MODE == EN_C) {   // over each half warp, then over the warps, in a fixed order
+    __shared__ double red[4][2][13];
 #pragma unroll
-      for (int t = 0; t < 22; ++t) a.part[(long long)u.slot * 22 + t] = acc[t];
+    for (int o = 8; o > 0; o >>= 1) {
+#pragma unroll
+      for (int p = 0; p < 12; ++p) acc[p] += __shfl_xor_sync(0xffffffffu, acc[p], o);
+      rsum += __shfl_xor_sync(0xffffffffu, rsum, o);
+    }
+    if (lane16 == 0) {
+#pragma unroll
+      for (int p = 0; p < 12; ++p) red[warp][half][p] = acc[p];
+      red[warp][half][12] = rsum;
+    }
+    __syncthreads();
+    if (threadIdx.x < 25) {   // 0-11: half 0's pairs and the density; 12-20: half 1's
+      const int t = threadIdx.x, hf = t >= 13, p = t < 13 ? t : t - 13;
+      if (!hf || p < 9) {
+        double v = 0.0;
+        for (int w = 0; w < 4; ++w) v += red[w][hf][p];
+        a.part[su.sub * 22 + (p == 12 ? 21 : kEnergyPair[hf][p])] = v;
+      }
+    }
   }
 }
 
-// C^H of each cell from its energy partials (fixed order), one thread per (cell, pair).
+// C^H of each cell from its energy partials, one warp per (cell, pair), lanes
+// over the sub-slots and a shuffle tree (fixed order).  One thread per pair
+// chased the slots one load after another: 564 us at 192^3.
 __global__ void k_energy_fin(const CellDesc* cells, const int* slot_begin, const int* slot_end,
-                             const double* part, double* C, double* dens, int ncells) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+                             const double* part, double* C, double* dens, int ncells, int nsub) {
+  const int t = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (t >= ncells * 22) return;
   const int cell = t / 22, q = t % 22;
   const CellDesc cd = cells[cell];
   const double nvx = (double)cd.nx * cd.ny * cd.nz;
   const double vol = nvx * cd.h * cd.h * cd.h;
   double s = 0.0;
-  for (int sl = slot_begin[cell]; sl < slot_end[cell]; ++sl) s += part[(long long)sl * 22 + q];
+  const long long end = (long long)slot_end[cell] * nsub;
+#pragma unroll 4
+  for (long long sl = (long long)slot_begin[cell] * nsub + lane; sl < end; sl += 32) s += part[sl * 22 + q];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane != 0) return;
   if (q == 21) {
     dens[cell] = s / nvx;
     return;

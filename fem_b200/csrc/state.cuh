@@ -182,11 +182,12 @@ struct femh_handle {
   size_t part_g_slots = 0;      // slots of level 0 before any compaction (units keep their slot)
   int bsub = 1;                 // block PCG update / direction: CTAs per level-0 node unit
   int bsub_g = 1;               // block PCG Gram kernels: CTAs per level-0 node unit
+  int bsub_e = 1;               // energy kernels: CTAs per level-0 node unit
   std::vector<CGState> state;
   double* d_part_s = nullptr;   // stencil partials [slots][6]
   double* d_part_n = nullptr;   // node partials [slots][6][2]
   double* d_part_z = nullptr;   // node partials [slots][6]
-  double* d_part_e = nullptr;   // energy partials [slots][21]
+  double* d_part_e = nullptr;   // energy partials [sub-slots][22]; load sums [slots][6][3] before the solve
   double* d_C = nullptr;        // [ncells][36]
   double* d_W = nullptr;        // [ncells][21]
   double* d_stage = nullptr;    // output staging (dCdrho, fields, apply), allocated on first use
