@@ -6,6 +6,7 @@
 // SamplesGenerator/NumericalCoarseningUsingMultiGrid.cpp:221-345.  There is no
 // CPU fallback: every numeric step below is one of this library's kernels.
 #include "kernels.cuh"
+#include "tail.cuh"
 #include "state.cuh"
 
 namespace {
@@ -502,6 +503,34 @@ double cell_setup_bytes(const femh_config& c, int nx, int ny, int nz) {
   return b;
 }
 
+// First level of the V-cycle's fused end (tail.cuh): the finest level below 0
+// on which every cell's vectors fit one CTA's shared memory (12^3 nodes in
+// FP32, 10^3 in FP64), while its CTAs -- one per cell and load case, one per
+// multiprocessor -- stay within eight waves; beyond that the level kernels,
+// which spread a level over all multiprocessors, are the faster ones again.
+constexpr int kTailSmem = 220 * 1024;
+int tail_level(const femh_handle* H, size_t msz) {
+  const int nlev = (int)H->levels.size();
+  if (H->cfg.pre_smooth > 8 || H->cfg.post_smooth > 8) return nlev;
+  for (int l = 1; l < nlev; ++l) {
+    const Level& L = H->levels[l];
+    if (nlev - l > kTailLevels || (long long)L.cells.size() * kNumRhs > 8LL * H->nsm) continue;
+    bool fits = true;
+    for (const CellDesc& c0 : L.cells) {
+      int n[kTailLevels], nl = 0;
+      const CellDesc* c = &c0;
+      for (int q = l;; ++q) {
+        n[nl++] = c->nx * c->ny * c->nz;
+        if (c->child < 0) break;
+        c = &H->levels[q + 1].cells[c->child];
+      }
+      fits = fits && tail_values(n, nl) * (long long)msz <= kTailSmem;
+    }
+    if (fits) return l;
+  }
+  return nlev;
+}
+
 void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vector<double>& hs) {
   const femh_config& c = H->cfg;
   const bool mixed = c.precision == FEMH_MIXED;
@@ -655,10 +684,15 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
       }
       L.d_coarse_list = upload(ar, L.coarse_list, s);
       L.d_aoff = upload(ar, aoff, s);
+      std::vector<long long> cell_aoff(L.cells.size(), -1);
+      for (size_t q = 0; q < L.coarse_list.size(); ++q) cell_aoff[L.coarse_list[q]] = aoff[q];
+      L.d_cell_aoff = upload(ar, cell_aoff, s);
+      CK(cudaStreamSynchronize(s));   // local vectors go out of scope
       L.d_A = ar.arr<double>(o);
       L.d_Awork = ar.arr<double>(o);
     }
   }
+  H->tail = gmg ? tail_level(H, msz) : nlev;
   // ---- fine-level arrays
   const long long nv = H->nvox;
   H->rho_in = ar.arr<double>(nv);
@@ -889,7 +923,7 @@ void autotune_level0_fp64(femh_handle* H) {
 template <typename T>
 void autotune_levels(femh_handle* H, bool mg) {
   cudaStream_t s = H->stream;
-  for (size_t l = 0; l < H->levels.size(); ++l) {
+  for (size_t l = 0; l < (size_t)H->tail; ++l) {   // (the fused end has nothing to tune)
     Level& L = H->levels[l];
     const bool smooth = mg && l > 0;   // coarse levels only run smoothing sweeps
     if ((smooth ? L.smooth.su : L.all.su).empty()) continue;
@@ -1098,7 +1132,7 @@ void vcycle_level_down(femh_handle* H, int l, const TB* b, TM* cur, TM* oth, TM*
   }
   stencil<TM, OUT_RESID>(H, L, true, (const TM*)cur, oth, b, (const TMC*)L.kc, nullptr, stt, w[0]);
   Level& C = H->levels[l + 1];
-  const bool c_smooth = !C.smooth.su.empty();   // also C's first sweep from a zero guess
+  const bool c_smooth = !C.smooth.su.empty() && l + 1 < H->tail;   // also C's first sweep from a zero guess
   Prof prof_(H, level_name(H, "k_restrict", l),
              18.0 * sizeof(TM) * (L.nodes_smooth + C.ntot) + (c_smooth ? (18.0 * sizeof(TM) + (C.binv ? 24.0 : 4.0)) * C.nodes_smooth : 0.0));
   k_restrict<TM, TM><<<NODE_GRID(C.all), 256, 0, s>>>(L.d_cells, C.d_cells, C.all.d_nu, oth, (TM*)C.bv,
@@ -1130,6 +1164,48 @@ void vcycle_level_up(femh_handle* H, int l, const TB* b, TM* x, TM* t, const TM*
   }
 }
 
+// The fused end of the V-cycle: levels H->tail and below, right-hand side in
+// the tail level's bv, solution to x.
+template <typename TM, typename TMC>
+void vcycle_tail(femh_handle* H, TM* x) {
+  const int l0 = H->tail, nlev = (int)H->levels.size();
+  TailArgs a{};
+  size_t smem = 0;
+  for (int l = l0; l < nlev; ++l) {
+    const Level& L = H->levels[l];
+    a.lev[l - l0] = TailLevel{L.d_cells, L.kc, L.invd, L.binv, L.d_A, L.d_cell_aoff};
+  }
+  Level& T = H->levels[l0];
+  for (const CellDesc& c0 : T.cells) {
+    int n[kTailLevels], nl = 0;
+    const CellDesc* c = &c0;
+    for (int q = l0;; ++q) {
+      n[nl++] = c->nx * c->ny * c->nz;
+      if (c->child < 0) break;
+      c = &H->levels[q + 1].cells[c->child];
+    }
+    smem = std::max(smem, (size_t)tail_values(n, nl) * sizeof(TM));
+  }
+  a.b = T.bv;
+  a.x = x;
+  a.ntot = T.ntot;
+  a.stt = H->d_state;
+  a.k = H->hk;
+  a.pre = H->cfg.pre_smooth;
+  a.post = H->cfg.post_smooth;
+  for (int q = 0; q < a.pre; ++q) a.w_pre[q] = H->w_pre[q];
+  for (int q = 0; q < a.post; ++q) a.w_post[q] = H->w_post[q];
+  auto fn = k_tail<TM, TMC>;
+  static bool attr = false;
+  if (!attr) {
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
+    attr = true;
+  }
+  Prof prof_(H, "k_tail", 36.0 * sizeof(TM) * (double)T.ntot);
+  fn<<<dim3((unsigned)T.cells.size(), kNumRhs), kTailThreads, smem, H->stream>>>(a);
+  LAUNCH_CHECK(H);
+}
+
 // dot_part != nullptr: the last level-0 sweep writes the z . r0 partials
 // there (per stencil unit slot).
 template <typename TM, typename TMC, typename TR>
@@ -1146,12 +1222,13 @@ TM* vcycle(femh_handle* H, const TR* r0, double* dot_part) {
     tmp[l] = oth;
     sol[l] = (c.post_smooth % 2 == 0) ? cur : oth;
   }
-  for (int l = 0; l < nlev; ++l) {
+  for (int l = 0; l < H->tail; ++l) {
     if (l == 0) vcycle_level_down<TM, TMC, TR>(H, 0, r0, (TM*)H->levels[0].xa, (TM*)H->levels[0].xb, sol[0]);
     else vcycle_level_down<TM, TMC, TM>(H, l, (const TM*)H->levels[l].bv, (TM*)H->levels[l].xa,
                                          (TM*)H->levels[l].xb, sol[l]);
   }
-  for (int l = nlev - 2; l >= 0; --l) {
+  if (H->tail < nlev) vcycle_tail<TM, TMC>(H, sol[H->tail]);
+  for (int l = std::min(nlev - 2, H->tail - 1); l >= 0; --l) {
     if (l == 0) vcycle_level_up<TM, TMC, TR>(H, 0, r0, sm[0], tmp[0], sol[1], dot_part);
     else vcycle_level_up<TM, TMC, TM>(H, l, (const TM*)H->levels[l].bv, sm[l], tmp[l], sol[l + 1], nullptr);
   }

@@ -122,6 +122,7 @@ struct Level {
   std::vector<int> coarse_list;                  // cells whose coarsest level this is
   int* d_coarse_list = nullptr;
   long long* d_aoff = nullptr;
+  long long* d_cell_aoff = nullptr;              // the same by cell (coarsest cells of this level)
   double* d_A = nullptr;
   double* d_Awork = nullptr;
   int coarse_maxm = 0;
@@ -158,6 +159,7 @@ struct femh_handle {
   int prec_key = -1, solver_key = -1, bf16_key = -1;
   Arena setup;
   std::vector<Level> levels;
+  int tail = 0;                 // first level of the fused coarse end of the V-cycle (levels.size(): none)
   std::map<std::string, int> tune_cache;   // autotuned x-chunk per level signature
   int ncells = 0;
   std::vector<long long> cell_vox;   // voxels per cell
