@@ -1296,7 +1296,7 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
   block_gram<true, TP, TV>(H, "k_bgram_pq", (const TP*)p, (const TV*)q, part_a);
   {
     Prof prof_(H, "k_bfin_alpha", 0.0);
-    k_bfin_alpha<<<nc, 256, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, part_a, nc, block_drop<TM>(), nsub_g);
+    k_bfin_alpha<<<nc, 1024, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, part_a, nc, block_drop<TM>(), nsub_g);
     LAUNCH_CHECK(H);
   }
   {
@@ -1312,7 +1312,7 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
   block_gram<false, TV, TM>(H, "k_bgram_qz", (const TV*)q, (const TM*)z, part_b);
   {
     Prof prof_(H, "k_bfin_beta", 0.0);
-    k_bfin_beta<<<nc, 256, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_b, part_a, part_b, nc,
+    k_bfin_beta<<<nc, 1024, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_b, part_a, part_b, nc,
                                    block_drop<TM>(), nsub_g, nsub);
     LAUNCH_CHECK(H);
   }
@@ -1446,7 +1446,7 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
       block_gram<false, TM, TV>(H, "k_bgram_zr", (const TM*)z, (const TV*)r, H->d_part_g);
       {
         Prof prof_(H, "k_bfin_rz", 0.0);
-        k_bfin_rz<<<nc, 256, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_g, nc, H->bsub_g);
+        k_bfin_rz<<<nc, 1024, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_g, nc, H->bsub_g);
         LAUNCH_CHECK(H);
       }
       {

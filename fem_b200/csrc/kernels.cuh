@@ -374,60 +374,52 @@ constexpr int kBlockStallWindow = 200;
 // Index of (i, j), i <= j, in the 21 upper-triangle entries of a 6x6 matrix.
 __host__ __device__ constexpr int sym6(int i, int j) { return i * 6 - i * (i - 1) / 2 + (j - i); }
 
-// G X = s B (6x6, row-major) by Cholesky on the columns in mask, a column
-// with a pivot below drop times its diagonal dropped (its row of X is 0).
-// Returns false if a pivot is below -1e-8 times its diagonal (G indefinite
-// beyond rounding), not finite, or no column is kept.
-__device__ __noinline__ bool chol_solve6(const double* __restrict__ G, const double* __restrict__ B, double sgn,
-                                         double* __restrict__ X, int mask, double drop) {
-  double L[6][6];
-  int keep = 0;
-  bool ok = true;
+// G X = s B (6x6, row-major, shared memory) by Cholesky on the columns in mask,
+// a column with a pivot below drop times its diagonal dropped (its row of X is
+// 0).  Returns false if a pivot is below -1e-8 times its diagonal (G indefinite
+// beyond rounding), not finite, or no column is kept.  One warp: lane r holds
+// row r of L (r < 6), then lane c solves column c; one thread alone took 10 us
+// of divisions in a row, the warp takes ~1.
+__device__ __forceinline__ bool chol_solve6(const double* G, const double* B, double sgn, double* X, int mask,
+                                            double drop) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, r = min(lane, 5);
+  double l[6], inv[6];
+  bool ok = true, any = false;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
-    const double gkk = G[k * 6 + k];
-    double d = gkk;
+    double v = G[r * 6 + k];
 #pragma unroll
-    for (int j = 0; j < k; ++j)
-      if (keep >> j & 1) d -= L[k][j] * L[k][j];
+    for (int j = 0; j < k; ++j) v -= l[j] * __shfl_sync(full, l[j], k);
+    const double d = __shfl_sync(full, v, k), gkk = G[k * 6 + k];
     const bool in = mask >> k & 1;
     if (in && (!isfinite(d) || d < -1e-8 * fabs(gkk))) ok = false;
     const bool use = in && gkk > 0.0 && d > drop * gkk;
     const double lkk = use ? sqrt(d) : 1.0;
-    L[k][k] = lkk;
+    inv[k] = use ? 1.0 / lkk : 0.0;
+    l[k] = r == k ? lkk : (r > k ? v * inv[k] : 0.0);
+    any = any || use;
+  }
+  double y[6];
 #pragma unroll
-    for (int i = k + 1; i < 6; ++i) {
-      double v = G[i * 6 + k];
+  for (int k = 0; k < 6; ++k) {
+    double v = sgn * B[k * 6 + r];
 #pragma unroll
-      for (int j = 0; j < k; ++j)
-        if (keep >> j & 1) v -= L[i][j] * L[k][j];
-      L[i][k] = use ? v / lkk : 0.0;
-    }
-    if (use) keep |= 1 << k;
+    for (int j = 0; j < k; ++j) v -= __shfl_sync(full, l[j], k) * y[j];
+    y[k] = v * inv[k];
   }
 #pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    double y[6], x[6];
+  for (int k = 5; k >= 0; --k) {
+    double v = y[k];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      double v = sgn * B[k * 6 + c];
-#pragma unroll
-      for (int j = 0; j < k; ++j)
-        if (keep >> j & 1) v -= L[k][j] * y[j];
-      y[k] = (keep >> k & 1) ? v / L[k][k] : 0.0;
-    }
-#pragma unroll
-    for (int k = 5; k >= 0; --k) {
-      double v = y[k];
-#pragma unroll
-      for (int j = k + 1; j < 6; ++j)
-        if (keep >> j & 1) v -= L[j][k] * x[j];
-      x[k] = (keep >> k & 1) ? v / L[k][k] : 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) X[k * 6 + c] = x[k];
+    for (int j = k + 1; j < 6; ++j) v -= __shfl_sync(full, l[k], j) * y[j];
+    y[k] = v * inv[k];
   }
-  return ok && keep != 0;
+  if (lane < 6)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) X[k * 6 + lane] = y[k];
+  __syncwarp();
+  return ok && any;
 }
 
 // The block kernels split each node unit into S sub-ranges, one CTA each (S
@@ -489,56 +481,56 @@ k_bgram(const CellDesc* cells, const NodeUnit* units, const TA* __restrict__ a, 
     for (int k = 0; k < NV; ++k) part[su.sub * NV + k] = v[k];
 }
 
-// Sum of a cell's per-slot partials over its slot range [b, e) by a
-// 256-thread CTA in a fixed order (deterministic): thread t adds value
-// t % NV of the slots b + t / NV, b + t / NV + G, ... (G = 256 / NV groups,
-// coalesced rows), then thread k < NV adds the G group sums of value k.
-// out[k] (shared memory) is valid after the call in every thread.
-template <int NV>
-__device__ __forceinline__ void cta_sum_slots(const double* __restrict__ part, int b, int e, double* red,
-                                              double* out) {
-  constexpr int G = 256 / NV;
-  const int t = threadIdx.x, k = t % NV, grp = t / NV;
-  if (grp < G) {
+// Sums of a cell's per-slot partials by a 1024-thread CTA in a fixed order
+// (deterministic): value v of set q (NQ sets of n[q] values, slots [b[q], e[q])
+// of part[q]) is added up by G thread groups, group g over the slots b + g,
+// b + g + G, ... (coalesced rows, eight loads in flight per thread), then the G
+// group sums by one thread.  out[v] (shared memory, the sets one after another)
+// is valid after the call in every thread.  256 threads without the unrolling
+// took 24 us of a 128^3 iteration for the three sums of the beta step.
+template <int NQ, int NV>
+__device__ __forceinline__ void cta_sums(const double* const (&part)[NQ], const int (&n)[NQ], const int (&b)[NQ],
+                                         const int (&e)[NQ], double* red, double* out) {
+  constexpr int G = 1024 / NV;
+  const int t = threadIdx.x, v = t % NV, g = t / NV;
+  if (g < G) {
+    int q = 0, w = v;
+    while (q + 1 < NQ && w >= n[q]) w -= n[q++];
+    const double* p = part[q] + w;
+    const int nq = n[q], end = e[q];
     double acc = 0.0;
-    for (int sl = b + grp; sl < e; sl += G) acc += part[(long long)sl * NV + k];
-    red[grp * NV + k] = acc;
+#pragma unroll 8
+    for (int sl = b[q] + g; sl < end; sl += G) acc += p[(long long)sl * nq];
+    red[g * NV + v] = acc;
   }
   __syncthreads();
   if (t < NV) {
     double acc = 0.0;
+#pragma unroll 8
     for (int g2 = 0; g2 < G; ++g2) acc += red[g2 * NV + t];
     out[t] = acc;
   }
   __syncthreads();
 }
 
-// Full 6x6 matrix from 21 upper-triangle values (sym) or 36 row-major ones.
-__device__ __forceinline__ void expand6(const double* v, bool sym, double* M) {
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j) M[i * 6 + j] = sym ? v[i <= j ? sym6(i, j) : sym6(j, i)] : v[i * 6 + j];
-}
-
-// The block stops: its load cases leave the loop with `status`.
-__device__ void block_stop(BlockCG& B, CGState* stt, int cell, int status) {
-  B.live = 0;
-#pragma unroll 1
-  for (int j = 0; j < kNumRhs; ++j)
-    if (B.mask >> j & 1) {
-      CGState& S = stt[cell * kNumRhs + j];
-      S.active = 0;
-      S.status = status == CG_MAXITER && S.rel < S.tol ? CG_CONVERGED : status;
-    }
+// The block stops: its load cases leave the loop with `status`.  One warp.
+__device__ __forceinline__ void block_stop(BlockCG& B, CGState* stt, int cell, int mask, int status) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) B.live = 0;
+  if (lane < kNumRhs && (mask >> lane & 1)) {
+    CGState& S = stt[cell * kNumRhs + lane];
+    S.active = 0;
+    S.status = status == CG_MAXITER && S.rel < S.tol ? CG_CONVERGED : status;
+  }
 }
 
 // z_j . r_j of every load case of the block positive: the preconditioner is
-// positive on the current residuals.
+// positive on the current residuals.  One warp.
 __device__ __forceinline__ bool zr_positive(const double* Z, int mask) {
-  bool ok = true;
-#pragma unroll
-  for (int j = 0; j < 6; ++j)
-    if (mask >> j & 1) ok = ok && Z[j * 7] > 0.0 && isfinite(Z[j * 7]);
-  return ok;
+  const int lane = threadIdx.x & 31;
+  const bool mine = lane < kNumRhs && (mask >> lane & 1);
+  const double z = mine ? Z[lane * 7] : 1.0;
+  return __all_sync(0xffffffffu, z > 0.0 && isfinite(z));
 }
 
 // After k_fin_init: the block of each cell is its live load cases.
@@ -557,81 +549,96 @@ __global__ void k_binit(BlockCG* bst, const CGState* stt, int ncells) {
 }
 
 // After the first preconditioner application: Z^T R of the start (beta = 0).
-// One 256-thread CTA per cell.
-__global__ void __launch_bounds__(256) k_bfin_rz(BlockCG* bst, CGState* stt, const int* sb, const int* se,
-                                                 const double* part_zr, int ncells, int nsub) {
-  const int cell = blockIdx.x;
+// One 1024-thread CTA per cell.
+__global__ void __launch_bounds__(1024) k_bfin_rz(BlockCG* bst, CGState* stt, const int* sb, const int* se,
+                                                  const double* part_zr, int ncells, int nsub) {
+  const int cell = blockIdx.x, lane = threadIdx.x;
   BlockCG& B = bst[cell];
   if (!B.live) return;
-  __shared__ double red[256], Z[36];
-  cta_sum_slots<36>(part_zr, sb[cell] * nsub, se[cell] * nsub, red, Z);
-  if (threadIdx.x != 0) return;
-  if (!zr_positive(Z, B.mask)) return block_stop(B, stt, cell, CG_BLOCK_FAIL);
-  for (int k = 0; k < 36; ++k) B.zr[k] = Z[k];
+  __shared__ double red[1024], Z[36];
+  cta_sums<1, 36>({part_zr}, {36}, {sb[cell] * nsub}, {se[cell] * nsub}, red, Z);
+  if (lane >= 32) return;
+  if (!zr_positive(Z, B.mask)) return block_stop(B, stt, cell, B.mask, CG_BLOCK_FAIL);
+  for (int k = lane; k < 36; k += 32) B.zr[k] = Z[k];
 }
 
-// G = P^T K P, alpha = G^+ Z^T R.  One 256-thread CTA per cell.
-__global__ void __launch_bounds__(256) k_bfin_alpha(BlockCG* bst, CGState* stt, const int* sb, const int* se,
-                                                    const double* part_g, int ncells, double drop, int nsub) {
-  const int cell = blockIdx.x;
+// G = P^T K P, alpha = G^+ Z^T R.  One 1024-thread CTA per cell.
+__global__ void __launch_bounds__(1024) k_bfin_alpha(BlockCG* bst, CGState* stt, const int* sb, const int* se,
+                                                     const double* part_g, int ncells, double drop, int nsub) {
+  const int cell = blockIdx.x, lane = threadIdx.x;
   BlockCG& B = bst[cell];
   if (!B.live) return;
-  __shared__ double red[256], g[21], G[36], A[36], ZR[36];
-  cta_sum_slots<21>(part_g, sb[cell] * nsub, se[cell] * nsub, red, g);
-  if (threadIdx.x < 36) ZR[threadIdx.x] = B.zr[threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  expand6(g, true, G);
-  if (!chol_solve6(G, ZR, 1.0, A, B.mask, drop)) return block_stop(B, stt, cell, CG_BLOCK_FAIL);
-  for (int k = 0; k < 36; ++k) {
+  __shared__ double red[1024], g[21], G[36], A[36], ZR[36];
+  cta_sums<1, 21>({part_g}, {21}, {sb[cell] * nsub}, {se[cell] * nsub}, red, g);
+  if (lane >= 32) return;
+  for (int k = lane; k < 36; k += 32) {
+    const int i = k / 6, j = k % 6;
+    G[k] = g[i <= j ? sym6(i, j) : sym6(j, i)];
+    ZR[k] = B.zr[k];
+  }
+  __syncwarp();
+  if (!chol_solve6(G, ZR, 1.0, A, B.mask, drop)) return block_stop(B, stt, cell, B.mask, CG_BLOCK_FAIL);
+  for (int k = lane; k < 36; k += 32) {
     B.alpha[k] = A[k];
     B.g[k] = G[k];
   }
 }
 
 // After the update and the preconditioner: convergence of every load case of
-// the block, then beta = -G^+ (K P)^T Z.  One 256-thread CTA per cell; the
+// the block, then beta = -G^+ (K P)^T Z.  One 1024-thread CTA per cell; the
 // Gram partials come in nsub_g sub-slots per slot, the ||r||^2 ones in nsub.
-__global__ void __launch_bounds__(256) k_bfin_beta(BlockCG* bst, CGState* stt, const int* sb, const int* se,
-                                                   const double* part_upd, const double* part_zr,
-                                                   const double* part_qz, int ncells, double drop, int nsub_g,
-                                                   int nsub) {
-  const int cell = blockIdx.x;
+__global__ void __launch_bounds__(1024) k_bfin_beta(BlockCG* bst, CGState* stt, const int* sb, const int* se,
+                                                    const double* part_upd, const double* part_zr,
+                                                    const double* part_qz, int ncells, double drop, int nsub_g,
+                                                    int nsub) {
+  const int cell = blockIdx.x, lane = threadIdx.x;
   BlockCG& B = bst[cell];
   if (!B.live) return;
-  const int b = sb[cell] * nsub_g, e = se[cell] * nsub_g;
-  __shared__ double red[256], Z[36], Q[36], T[36], G[36], rr[kNumRhs];
-  cta_sum_slots<36>(part_zr, b, e, red, Z);
-  cta_sum_slots<36>(part_qz, b, e, red, Q);
-  cta_sum_slots<kNumRhs>(part_upd, sb[cell] * nsub, se[cell] * nsub, red, rr);
-  if (threadIdx.x < 36) G[threadIdx.x] = B.g[threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  bool all = true, spent = false, bad = false;
-  double worst = 0.0;
-  for (int j = 0; j < kNumRhs; ++j) {
-    if (!(B.mask >> j & 1)) continue;
-    CGState& S = stt[cell * kNumRhs + j];
-    S.rr = rr[j];
+  const int b = sb[cell], e = se[cell];
+  __shared__ double red[1024], sums[78], T[36], G[36];
+  cta_sums<3, 78>({part_zr, part_qz, part_upd}, {36, 36, kNumRhs}, {b * nsub_g, b * nsub_g, b * nsub},
+                  {e * nsub_g, e * nsub_g, e * nsub}, red, sums);
+  if (lane >= 32) return;
+  const double *Z = sums, *Q = sums + 36, *rr = sums + 72;
+  const unsigned full = 0xffffffffu;
+  const int mask = B.mask;
+  const bool mine = lane < kNumRhs && (mask >> lane & 1);
+  double rel = 0.0;
+  bool conv = true, spent = false, bad = false;
+  if (mine) {
+    CGState& S = stt[cell * kNumRhs + lane];
+    rel = sqrt(rr[lane] / S.bnorm2);
+    S.rr = rr[lane];
     S.iters += 1;
-    S.rel = sqrt(S.rr / S.bnorm2);
-    all = all && S.rel < S.tol;
-    spent = spent || S.iters >= S.max_iter;
-    bad = bad || !isfinite(S.rel);
-    worst = fmax(worst, S.rel);
+    S.rel = rel;
+    conv = rel < S.tol;
+    spent = S.iters >= S.max_iter;
+    bad = !isfinite(rel);
   }
-  if (all) return block_stop(B, stt, cell, CG_CONVERGED);
-  if (bad) return block_stop(B, stt, cell, CG_BREAKDOWN);
-  if (spent) return block_stop(B, stt, cell, CG_MAXITER);
-  if (worst < 0.5 * B.best) {
-    B.best = worst;
-    B.since = 0;
-  } else if (++B.since >= kBlockStallWindow) {
-    return block_stop(B, stt, cell, CG_BLOCK_FAIL);
+  if (__all_sync(full, conv)) return block_stop(B, stt, cell, mask, CG_CONVERGED);
+  if (__any_sync(full, bad)) return block_stop(B, stt, cell, mask, CG_BREAKDOWN);
+  if (__any_sync(full, spent)) return block_stop(B, stt, cell, mask, CG_MAXITER);
+  double worst = rel;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) worst = fmax(worst, __shfl_xor_sync(full, worst, o));
+  worst = __shfl_sync(full, worst, 0);
+  const double best = B.best;
+  const int since = B.since + 1;
+  __syncwarp();
+  if (worst < 0.5 * best) {
+    if (lane == 0) {
+      B.best = worst;
+      B.since = 0;
+    }
+  } else {
+    if (lane == 0) B.since = since;
+    if (since >= kBlockStallWindow) return block_stop(B, stt, cell, mask, CG_BLOCK_FAIL);
   }
-  if (!zr_positive(Z, B.mask) || !chol_solve6(G, Q, -1.0, T, B.mask, drop))
-    return block_stop(B, stt, cell, CG_BLOCK_FAIL);
-  for (int k = 0; k < 36; ++k) {
+  for (int k = lane; k < 36; k += 32) G[k] = B.g[k];
+  __syncwarp();
+  if (!zr_positive(Z, mask) || !chol_solve6(G, Q, -1.0, T, mask, drop))
+    return block_stop(B, stt, cell, mask, CG_BLOCK_FAIL);
+  for (int k = lane; k < 36; k += 32) {
     B.beta[k] = T[k];
     B.zr[k] = Z[k];
   }
