@@ -717,15 +717,17 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
   H->d_part_s = ar.arr<double>(std::max(L0.all.su.size(), L0.su64.size()) * kNumRhs);
   H->d_part_n = ar.arr<double>(L0.all.nu.size() * kNumRhs * 2);
   H->part_g_slots = L0.all.nu.size();
-  // CTAs per level-0 node unit in the block PCG's kernels.  The update and
-  // direction kernels (three 256-thread CTAs per SM) get >= 16 CTAs per SM, so
-  // the last wave is a small part of the launch (128^3: 1024 units -> 4096
-  // CTAs; ncu showed 1024 CTAs in 2.3 waves at 23-33% of the SMs' warps);
-  // the Gram kernels only enough for two per SM, because every extra CTA adds
-  // 21-36 partial sums that the per-cell finalisation reads back.
+  // CTAs per level-0 node unit (2048 nodes) in the block PCG's kernels.  The
+  // update and direction kernels get >= 16 CTAs per SM as long as every thread
+  // of a 256-thread CTA has a node (8 CTAs per unit): 32 CTAs per unit left three
+  // quarters of their threads without one (64^3 update 163 us, of 270 MB).
+  // Cells too small to give every SM two such CTAs run 64-thread CTAs on 64
+  // nodes each.  The Gram kernels get only enough for two CTAs per SM, because
+  // every extra one adds partial sums that the per-cell finalisation reads back.
   const long long nsm = std::max(H->nsm, 1);
   H->bsub = H->bsub_g = 1;
-  while (H->bsub < 32 && (long long)H->part_g_slots * H->bsub < 16 * nsm) H->bsub *= 2;
+  H->bt = (long long)H->part_g_slots * 8 < 2 * nsm ? 64 : 256;
+  while (H->bsub < 2048 / H->bt && (long long)H->part_g_slots * H->bsub < 16 * nsm) H->bsub *= 2;
   while (H->bsub_g < 32 && (long long)H->part_g_slots * H->bsub_g < 2 * nsm) H->bsub_g *= 2;
   H->d_part_g = ar.arr<double>(H->part_g_slots * H->bsub_g * 72);
   H->d_part_b = ar.arr<double>(H->part_g_slots * H->bsub * kNumRhs);
@@ -1303,8 +1305,9 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
     Prof prof_(H, "k_bupdate",
                18.0 * (5 * sizeof(TV) + sizeof(TP) + sizeof(TM) + (rm ? sizeof(TM) : 0)) * (double)L0.ntot +
                    (L0.binv ? 24.0 : 4.0) * (double)L0.ntot);
-    k_bupdate<TV, TP, TV, TM><<<grid, 256, 0, s>>>(L0.d_cells, L0.all.d_nu, x, r, p, q, L0.invd, (TM*)L0.xa, rm,
-                                                   H->w_pre[0], H->d_bcg, H->d_part_b, L0.ntot, L0.binv, nsub);
+    auto fn = H->bt == 64 ? k_bupdate<64, TV, TP, TV, TM> : k_bupdate<256, TV, TP, TV, TM>;
+    fn<<<grid, H->bt, 0, s>>>(L0.d_cells, L0.all.d_nu, x, r, p, q, L0.invd, (TM*)L0.xa, rm, H->w_pre[0], H->d_bcg,
+                              H->d_part_b, L0.ntot, L0.binv, nsub);
     LAUNCH_CHECK(H);
   }
   TM* z = vcycle_of<TM, TMC>(H, r, rm, nullptr);
@@ -1318,7 +1321,8 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
   }
   {
     Prof prof_(H, "k_bdir", 18.0 * (sizeof(TM) + 2 * sizeof(TP)) * (double)L0.ntot);
-    k_bdir<TP, TM><<<grid, 256, 0, s>>>(L0.d_cells, L0.all.d_nu, p, (const TM*)z, H->d_bcg, L0.ntot, 0, nsub);
+    auto fn = H->bt == 64 ? k_bdir<64, TP, TM> : k_bdir<256, TP, TM>;
+    fn<<<grid, H->bt, 0, s>>>(L0.d_cells, L0.all.d_nu, p, (const TM*)z, H->d_bcg, L0.ntot, 0, nsub);
     LAUNCH_CHECK(H);
   }
 }
@@ -1451,7 +1455,8 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
       }
       {
         Prof prof_(H, "k_bdir", 0.0);
-        k_bdir<TP, TM><<<dim3((unsigned)(L0.all.nu.size() * H->bsub)), 256, 0, s>>>(
+        auto fn = H->bt == 64 ? k_bdir<64, TP, TM> : k_bdir<256, TP, TM>;
+        fn<<<dim3((unsigned)(L0.all.nu.size() * H->bsub)), H->bt, 0, s>>>(
             L0.d_cells, L0.all.d_nu, p, (const TM*)z, H->d_bcg, L0.ntot, 1, H->bsub);
         LAUNCH_CHECK(H);
       }

@@ -647,10 +647,11 @@ __global__ void __launch_bounds__(1024) k_bfin_beta(BlockCG* bst, CGState* stt, 
 // X += P alpha, R -= Q alpha (Q = K P) for the load cases of each live block,
 // with ||r||^2 partials per load case ([sub-slot][6]) and, for the multigrid, the first
 // smoothing sweep z0 = omega D^-1 r and the residual copy rm of the V-cycle.
-// 256 threads; a node's new residuals wait in shared memory for the 3x3
-// node-block sweep (registers kept for three CTAs per SM: four measured slower).
-template <typename TV, typename TP, typename TQ, typename TZ>
-__global__ void __launch_bounds__(256, 3)
+// BT threads (256, or 64 where the cells are small: see bsub); a node's new
+// residuals wait in shared memory for the 3x3 node-block sweep (registers kept
+// for 768 threads per SM: 1024 measured slower).
+template <int BT, typename TV, typename TP, typename TQ, typename TZ>
+__global__ void __launch_bounds__(BT, 768 / BT)
 k_bupdate(const CellDesc* cells, const NodeUnit* units, TV* __restrict__ x, TV* __restrict__ r,
           const TP* __restrict__ p, const TQ* __restrict__ q, const float* __restrict__ invd, TZ* __restrict__ z0,
           TZ* __restrict__ rm, double omega, const BlockCG* bst, double* __restrict__ part, long long ntot,
@@ -659,7 +660,7 @@ k_bupdate(const CellDesc* cells, const NodeUnit* units, TV* __restrict__ x, TV* 
   const CellDesc cd = cells[su.u.cell];
   const int mask = bst[cd.id].live ? bst[cd.id].mask : 0;
   __shared__ double al[36];
-  __shared__ double rs[kNumRhs * 3][256];
+  __shared__ double rs[kNumRhs * 3][BT];
   if (threadIdx.x < 36) al[threadIdx.x] = bst[cd.id].alpha[threadIdx.x];
   __syncthreads();
   double v[kNumRhs];
@@ -717,8 +718,8 @@ k_bupdate(const CellDesc* cells, const NodeUnit* units, TV* __restrict__ x, TV* 
 }
 
 // P = Z + P beta for the load cases of each live block (first: P = Z).
-template <typename TP, typename TZ>
-__global__ void __launch_bounds__(256, 4)
+template <int BT, typename TP, typename TZ>
+__global__ void __launch_bounds__(BT, 1024 / BT)
 k_bdir(const CellDesc* cells, const NodeUnit* units, TP* __restrict__ p, const TZ* __restrict__ z,
        const BlockCG* bst, long long ntot, int first, int nsub) {
   const SubUnit su = sub_unit(units, nsub);

@@ -182,6 +182,7 @@ struct femh_handle {
   double* d_part_g = nullptr;   // block PCG 6x6 partials [2][sub-slots][36]
   double* d_part_b = nullptr;   // block PCG ||r||^2 partials [sub-slots][6]
   size_t part_g_slots = 0;      // slots of level 0 before any compaction (units keep their slot)
+  int bt = 256;                 // block PCG update / direction: threads per CTA
   int bsub = 1;                 // block PCG update / direction: CTAs per level-0 node unit
   int bsub_g = 1;               // block PCG Gram kernels: CTAs per level-0 node unit
   int bsub_e = 1;               // energy kernels: CTAs per level-0 node unit
