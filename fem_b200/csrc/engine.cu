@@ -1116,16 +1116,14 @@ const char* level_name(femh_handle* H, const char* base, int level) {
 template <typename TM, typename TMC, typename TB>
 void vcycle_level_down(femh_handle* H, int l, const TB* b, TM* cur, TM* oth, TM* sol) {
   const femh_config& c = H->cfg;
-  cudaStream_t s = H->stream;
   const std::vector<double>& w = H->w_pre;
   const CGState* stt = H->d_state;
   Level& L = H->levels[l];
   if (!L.coarse_list.empty()) {
     dim3 g((unsigned)L.coarse_list.size(), kNumRhs);
     Prof prof_(H, "k_coarse_solve", 0.0);
-    k_coarse_solve<TB, TM><<<g, 1024, sizeof(double) * L.coarse_maxm, s>>>(
-        L.d_cells, L.d_coarse_list, L.d_A, L.d_aoff, b, sol, stt, L.ntot);
-    LAUNCH_CHECK(H);
+    launch(H, k_coarse_solve<TB, TM>, g, 1024, sizeof(double) * L.coarse_maxm, L.d_cells, L.d_coarse_list, L.d_A,
+           L.d_aoff, b, sol, stt, L.ntot);
   }
   if (L.smooth.su.empty()) return;
   for (int sw = 1; sw < c.pre_smooth; ++sw) {
@@ -1137,25 +1135,21 @@ void vcycle_level_down(femh_handle* H, int l, const TB* b, TM* cur, TM* oth, TM*
   const bool c_smooth = !C.smooth.su.empty() && l + 1 < H->tail;   // also C's first sweep from a zero guess
   Prof prof_(H, level_name(H, "k_restrict", l),
              18.0 * sizeof(TM) * (L.nodes_smooth + C.ntot) + (c_smooth ? (18.0 * sizeof(TM) + (C.binv ? 24.0 : 4.0)) * C.nodes_smooth : 0.0));
-  k_restrict<TM, TM><<<NODE_GRID(C.all), 256, 0, s>>>(L.d_cells, C.d_cells, C.all.d_nu, oth, (TM*)C.bv,
-                                                      c_smooth ? (TM*)C.xa : (TM*)nullptr, C.invd, w[0], stt,
-                                                      L.ntot, C.ntot, C.binv);
-  LAUNCH_CHECK(H);
+  launch(H, k_restrict<TM, TM>, NODE_GRID(C.all), 256, 0, L.d_cells, C.d_cells, C.all.d_nu, oth, (TM*)C.bv,
+         c_smooth ? (TM*)C.xa : (TM*)nullptr, C.invd, w[0], stt, L.ntot, C.ntot, C.binv);
 }
 
 template <typename TM, typename TMC, typename TB>
 void vcycle_level_up(femh_handle* H, int l, const TB* b, TM* x, TM* t, const TM* coarse_sol, double* dot_part) {
   const femh_config& c = H->cfg;
-  cudaStream_t s = H->stream;
   const CGState* stt = H->d_state;
   Level& L = H->levels[l];
   if (L.smooth.su.empty()) return;
   Level& C = H->levels[l + 1];
   {
     Prof prof_(H, level_name(H, "k_prolong_add", l), 18.0 * sizeof(TM) * (2.0 * L.nodes_smooth + C.ntot));
-    k_prolong_add<TM, TM><<<NODE_GRID(L.smooth), 256, 0, s>>>(L.d_cells, C.d_cells, L.smooth.d_nu, x, coarse_sol,
-                                                              stt, L.ntot, C.ntot);
-    LAUNCH_CHECK(H);
+    launch(H, k_prolong_add<TM, TM>, NODE_GRID(L.smooth), 256, 0, L.d_cells, C.d_cells, L.smooth.d_nu, x, coarse_sol,
+           stt, L.ntot, C.ntot);
   }
   for (int sw = 0; sw < c.post_smooth; ++sw) {
     if (dot_part && sw + 1 == c.post_smooth)   // last sweep also forms z . b
@@ -1204,8 +1198,7 @@ void vcycle_tail(femh_handle* H, TM* x) {
     attr = true;
   }
   Prof prof_(H, "k_tail", 36.0 * sizeof(TM) * (double)T.ntot);
-  fn<<<dim3((unsigned)T.cells.size(), kNumRhs), kTailThreads, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
+  launch(H, fn, dim3((unsigned)T.cells.size(), kNumRhs), kTailThreads, smem, a);
 }
 
 // dot_part != nullptr: the last level-0 sweep writes the z . r0 partials
@@ -1268,9 +1261,7 @@ void block_gram(femh_handle* H, const char* name, const TA* a, const TB* b, doub
   Level& L0 = H->levels[0];
   const dim3 grid((unsigned)(L0.all.nu.size() * H->bsub_g));
   Prof prof_(H, name, 18.0 * (sizeof(TA) + sizeof(TB)) * (double)L0.ntot);
-  k_bgram<SYM, TA, TB><<<grid, 256, 0, H->stream>>>(L0.d_cells, L0.all.d_nu, a, b, H->d_bcg, part, L0.ntot,
-                                                    H->bsub_g);
-  LAUNCH_CHECK(H);
+  launch(H, k_bgram<SYM, TA, TB>, grid, 256, 0, L0.d_cells, L0.all.d_nu, a, b, H->d_bcg, part, L0.ntot, H->bsub_g);
 }
 
 // One block PCG iteration of the multigrid PCG (all live cells).
@@ -1280,7 +1271,6 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
   using TP = typename PR::P;
   using TM = typename PR::M;
   using TMC = typename PR::MC;
-  cudaStream_t s = H->stream;
   Level& L0 = H->levels[0];
   const int nc = H->ncells;
   const int nsub = H->bsub;
@@ -1298,32 +1288,28 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
   block_gram<true, TP, TV>(H, "k_bgram_pq", (const TP*)p, (const TV*)q, part_a);
   {
     Prof prof_(H, "k_bfin_alpha", 0.0);
-    k_bfin_alpha<<<nc, 1024, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, part_a, nc, block_drop<TM>(), nsub_g);
-    LAUNCH_CHECK(H);
+    launch(H, k_bfin_alpha, nc, 1024, 0, H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, part_a, nc, block_drop<TM>(), nsub_g);
   }
   {
     Prof prof_(H, "k_bupdate",
                18.0 * (5 * sizeof(TV) + sizeof(TP) + sizeof(TM) + (rm ? sizeof(TM) : 0)) * (double)L0.ntot +
                    (L0.binv ? 24.0 : 4.0) * (double)L0.ntot);
     auto fn = H->bt == 64 ? k_bupdate<64, TV, TP, TV, TM> : k_bupdate<256, TV, TP, TV, TM>;
-    fn<<<grid, H->bt, 0, s>>>(L0.d_cells, L0.all.d_nu, x, r, p, q, L0.invd, (TM*)L0.xa, rm, H->w_pre[0], H->d_bcg,
-                              H->d_part_b, L0.ntot, L0.binv, nsub);
-    LAUNCH_CHECK(H);
+    launch(H, fn, grid, H->bt, 0, L0.d_cells, L0.all.d_nu, x, r, p, q, L0.invd, (TM*)L0.xa, rm, H->w_pre[0],
+           H->d_bcg, H->d_part_b, L0.ntot, L0.binv, nsub);
   }
   TM* z = vcycle_of<TM, TMC>(H, r, rm, nullptr);
   block_gram<false, TM, TV>(H, "k_bgram_zr", (const TM*)z, (const TV*)r, part_a);
   block_gram<false, TV, TM>(H, "k_bgram_qz", (const TV*)q, (const TM*)z, part_b);
   {
     Prof prof_(H, "k_bfin_beta", 0.0);
-    k_bfin_beta<<<nc, 1024, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_b, part_a, part_b, nc,
-                                   block_drop<TM>(), nsub_g, nsub);
-    LAUNCH_CHECK(H);
+    launch(H, k_bfin_beta, nc, 1024, 0, H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_b, part_a, part_b, nc,
+           block_drop<TM>(), nsub_g, nsub);
   }
   {
     Prof prof_(H, "k_bdir", 18.0 * (sizeof(TM) + 2 * sizeof(TP)) * (double)L0.ntot);
     auto fn = H->bt == 64 ? k_bdir<64, TP, TM> : k_bdir<256, TP, TM>;
-    fn<<<grid, H->bt, 0, s>>>(L0.d_cells, L0.all.d_nu, p, (const TM*)z, H->d_bcg, L0.ntot, 0, nsub);
-    LAUNCH_CHECK(H);
+    launch(H, fn, grid, H->bt, 0, L0.d_cells, L0.all.d_nu, p, (const TM*)z, H->d_bcg, L0.ntot, 0, nsub);
   }
 }
 
@@ -1336,7 +1322,6 @@ void pcg_iteration(femh_handle* H, const typename PR::K* kcg, bool blk) {
   using TM = typename PR::M;
   using TMC = typename PR::MC;
   const femh_config& c = H->cfg;
-  cudaStream_t s = H->stream;
   Level& L0 = H->levels[0];
   const int nc = H->ncells;
   const bool gmg = c.solver == FEMH_GMG_PCG;
@@ -1350,18 +1335,15 @@ void pcg_iteration(femh_handle* H, const typename PR::K* kcg, bool blk) {
   {
     Prof prof_(H, "k_fin_alpha", 0.0);
     const bool l64 = sizeof(TV) == 8 && L0.use64;   // the apply above used the FP64 layout
-    k_fin_alpha<<<fin_blocks(nc), 128, 0, s>>>(stt, l64 ? L0.d_su64_sb : L0.d_su_sb,
-                                               l64 ? L0.d_su64_se : L0.d_su_se, H->d_part_s, nc);
-    LAUNCH_CHECK(H);
+    launch(H, k_fin_alpha, fin_blocks(nc), 128, 0, stt, l64 ? L0.d_su64_sb : L0.d_su_sb,
+           l64 ? L0.d_su64_se : L0.d_su_se, H->d_part_s, nc);
   }
   {
     Prof prof_(H, "k_cg_update",
                (18.0 * (5 * sizeof(TV) + sizeof(TP) + (gmg ? sizeof(TM) : 0) + (rm ? sizeof(TM) : 0)) + 4.0) *
                    (double)L0.ntot);
-    k_cg_update<TV, TP, TV, TM><<<NODE_GRID(L0.all), 256, 0, s>>>(
-        L0.d_cells, L0.all.d_nu, x, r, p, q, L0.invd, gmg ? (TM*)L0.xa : (TM*)nullptr, rm, H->w_pre[0], stt,
-        H->d_part_n, L0.ntot, L0.binv);
-    LAUNCH_CHECK(H);
+    launch(H, k_cg_update<TV, TP, TV, TM>, NODE_GRID(L0.all), 256, 0, L0.d_cells, L0.all.d_nu, x, r, p, q, L0.invd,
+           gmg ? (TM*)L0.xa : (TM*)nullptr, rm, H->w_pre[0], stt, H->d_part_n, L0.ntot, L0.binv);
   }
   TM* z = nullptr;
   const bool fuse = fuse_rz(H);
@@ -1370,22 +1352,18 @@ void pcg_iteration(femh_handle* H, const typename PR::K* kcg, bool blk) {
     z = vcycle_of<TM, TMC>(H, r, rm, dp);
     if (!fuse) {
       Prof prof_(H, "k_dot", 0.0);
-      k_dot<TM, TV><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, z, r, stt, H->d_part_z, L0.ntot);
-      LAUNCH_CHECK(H);
+      launch(H, k_dot<TM, TV>, NODE_GRID(L0.all), 256, 0, L0.d_cells, L0.all.d_nu, z, r, stt, H->d_part_z, L0.ntot);
     }
   }
   {
     Prof prof_(H, "k_fin_beta", 0.0);
-    k_fin_beta<<<fin_blocks(nc), 128, 0, s>>>(stt, L0.d_nu_sb, L0.d_nu_se, fuse ? L0.d_su_sb : L0.d_nu_sb,
-                                              fuse ? L0.d_su_se : L0.d_nu_se, H->d_part_n, H->d_part_z, nc,
-                                              gmg ? 0 : 1);
-    LAUNCH_CHECK(H);
+    launch(H, k_fin_beta, fin_blocks(nc), 128, 0, stt, L0.d_nu_sb, L0.d_nu_se, fuse ? L0.d_su_sb : L0.d_nu_sb,
+           fuse ? L0.d_su_se : L0.d_nu_se, H->d_part_n, H->d_part_z, nc, gmg ? 0 : 1);
   }
   {
     Prof prof_(H, "k_cg_dir", 18.0 * (sizeof(TM) + 2 * sizeof(TP)) * (double)L0.ntot);
-    k_cg_dir<TP, TM, TV><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, p, (const TM*)z,
-                                                           (const TV*)r, L0.invd, stt, L0.ntot);
-    LAUNCH_CHECK(H);
+    launch(H, k_cg_dir<TP, TM, TV>, NODE_GRID(L0.all), 256, 0, L0.d_cells, L0.all.d_nu, p, (const TM*)z,
+           (const TV*)r, L0.invd, stt, L0.ntot);
   }
 }
 
@@ -1456,9 +1434,8 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
       {
         Prof prof_(H, "k_bdir", 0.0);
         auto fn = H->bt == 64 ? k_bdir<64, TP, TM> : k_bdir<256, TP, TM>;
-        fn<<<dim3((unsigned)(L0.all.nu.size() * H->bsub)), H->bt, 0, s>>>(
-            L0.d_cells, L0.all.d_nu, p, (const TM*)z, H->d_bcg, L0.ntot, 1, H->bsub);
-        LAUNCH_CHECK(H);
+        launch(H, fn, dim3((unsigned)(L0.all.nu.size() * H->bsub)), H->bt, 0, L0.d_cells, L0.all.d_nu, p,
+               (const TM*)z, H->d_bcg, L0.ntot, 1, H->bsub);
       }
     }
   }
@@ -1468,8 +1445,7 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
     TM* z = vcycle_of<TM, TMC>(H, r, rm, dp);
     if (!fuse) {
       Prof prof_(H, "k_dot", 0.0);
-      k_dot<TM, TV><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, z, r, stt, H->d_part_z, L0.ntot);
-      LAUNCH_CHECK(H);
+      launch(H, k_dot<TM, TV>, NODE_GRID(L0.all), 256, 0, L0.d_cells, L0.all.d_nu, z, r, stt, H->d_part_z, L0.ntot);
     }
     {
       Prof prof_(H, "k_fin_rz", 0.0);
@@ -1479,9 +1455,8 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
     }
     {   // p = z (beta = 0; Jacobi z for pairs that fell back)
       Prof prof_(H, "k_cg_dir", 0.0);
-      k_cg_dir<TP, TM, TV><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, p, (const TM*)z,
-                                                             (const TV*)r, L0.invd, stt, L0.ntot);
-      LAUNCH_CHECK(H);
+      launch(H, k_cg_dir<TP, TM, TV>, NODE_GRID(L0.all), 256, 0, L0.d_cells, L0.all.d_nu, p, (const TM*)z,
+             (const TV*)r, L0.invd, stt, L0.ntot);
     }
   }
   const int chunk = H->prof ? 1 : std::max(1, c.graph_chunk > 0 ? c.graph_chunk : 8);
@@ -1534,8 +1509,7 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
     CK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     try {
       for (int i = 0; i < chunk; ++i) pcg_iteration<PR>(H, kcg, blk);
-      k_while_cond<<<1, 1024, 0, s>>>(cond, H->d_state, nc, listed, H->d_loop, chunk, limit);
-      LAUNCH_CHECK(H);
+      launch(H, k_while_cond, 1, 1024, 0, cond, H->d_state, nc, listed, H->d_loop, chunk, limit);
     } catch (...) {
       H->capturing = false;
       cudaGraph_t tmp = nullptr;

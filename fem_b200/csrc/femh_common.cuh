@@ -116,6 +116,18 @@ __device__ __forceinline__ void jacobi_dir(const float* __restrict__ binv, long 
   }
 }
 
+// First statement of every kernel of the CG loop: waits until the kernel before
+// it in the stream is complete and its writes are visible, then lets the next
+// one's CTAs be set up.  The loop's kernels are launched as programmatic
+// dependents (launch() in state.cuh), so a launch overlaps its predecessor's
+// run instead of following its end.  No kernel of the loop may return or touch
+// memory before this call: completion of one must imply completion of all
+// before it.
+__device__ __forceinline__ void griddep_sync() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Warp + block reduction of nv doubles; result valid in thread 0.
 template <int NV>
 __device__ __forceinline__ void block_reduce(double (&v)[NV], double* smem /* >= 32*NV */) {

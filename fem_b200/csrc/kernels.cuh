@@ -267,6 +267,7 @@ __global__ void k_cg_update(const CellDesc* cells, const NodeUnit* units, TV* __
                             const TQ* __restrict__ q, const float* __restrict__ invd, TZ* __restrict__ z0,
                             TZ* __restrict__ rm, double omega, const CGState* stt,
                             double* __restrict__ part, long long ntot, const float* __restrict__ binv) {
+  griddep_sync();
   const NodeUnit u = units[blockIdx.x];
   const int rhs = blockIdx.y;
   const CellDesc cd = cells[u.cell];
@@ -312,6 +313,7 @@ __global__ void k_cg_update(const CellDesc* cells, const NodeUnit* units, TV* __
 template <typename TP, typename TZ, typename TR>
 __global__ void k_cg_dir(const CellDesc* cells, const NodeUnit* units, TP* __restrict__ p, const TZ* __restrict__ zvec,
                          const TR* __restrict__ r, const float* __restrict__ invd, const CGState* stt, long long ntot) {
+  griddep_sync();
   const NodeUnit u = units[blockIdx.x];
   const int rhs = blockIdx.y;
   const CellDesc cd = cells[u.cell];
@@ -447,6 +449,7 @@ template <bool SYM, typename TA, typename TB>
 __global__ void __launch_bounds__(256, 2)
 k_bgram(const CellDesc* cells, const NodeUnit* units, const TA* __restrict__ a, const TB* __restrict__ b,
         const BlockCG* bst, double* __restrict__ part, long long ntot, int nsub) {
+  griddep_sync();
   constexpr int NV = SYM ? 21 : 36;
   const SubUnit su = sub_unit(units, nsub);
   const CellDesc cd = cells[su.u.cell];
@@ -565,6 +568,7 @@ __global__ void __launch_bounds__(1024) k_bfin_rz(BlockCG* bst, CGState* stt, co
 // G = P^T K P, alpha = G^+ Z^T R.  One 1024-thread CTA per cell.
 __global__ void __launch_bounds__(1024) k_bfin_alpha(BlockCG* bst, CGState* stt, const int* sb, const int* se,
                                                      const double* part_g, int ncells, double drop, int nsub) {
+  griddep_sync();
   const int cell = blockIdx.x, lane = threadIdx.x;
   BlockCG& B = bst[cell];
   if (!B.live) return;
@@ -591,6 +595,7 @@ __global__ void __launch_bounds__(1024) k_bfin_beta(BlockCG* bst, CGState* stt, 
                                                     const double* part_upd, const double* part_zr,
                                                     const double* part_qz, int ncells, double drop, int nsub_g,
                                                     int nsub) {
+  griddep_sync();
   const int cell = blockIdx.x, lane = threadIdx.x;
   BlockCG& B = bst[cell];
   if (!B.live) return;
@@ -656,6 +661,7 @@ k_bupdate(const CellDesc* cells, const NodeUnit* units, TV* __restrict__ x, TV* 
           const TP* __restrict__ p, const TQ* __restrict__ q, const float* __restrict__ invd, TZ* __restrict__ z0,
           TZ* __restrict__ rm, double omega, const BlockCG* bst, double* __restrict__ part, long long ntot,
           const float* __restrict__ binv, int nsub) {
+  griddep_sync();
   const SubUnit su = sub_unit(units, nsub);
   const CellDesc cd = cells[su.u.cell];
   const int mask = bst[cd.id].live ? bst[cd.id].mask : 0;
@@ -722,6 +728,7 @@ template <int BT, typename TP, typename TZ>
 __global__ void __launch_bounds__(BT, 1024 / BT)
 k_bdir(const CellDesc* cells, const NodeUnit* units, TP* __restrict__ p, const TZ* __restrict__ z,
        const BlockCG* bst, long long ntot, int first, int nsub) {
+  griddep_sync();
   const SubUnit su = sub_unit(units, nsub);
   const CellDesc cd = cells[su.u.cell];
   const int mask = bst[cd.id].live ? bst[cd.id].mask : 0;
@@ -810,6 +817,7 @@ __global__ void k_fin_rz(CGState* stt, const int* slot_begin, const int* slot_en
 // alpha = rz / (p . K p); breakdown if p.Kp <= 0 or not finite.
 __global__ void k_fin_alpha(CGState* stt, const int* slot_begin, const int* slot_end,
                             const double* part, int ncells) {
+  griddep_sync();
   FIN_PROLOGUE
   CGState S = stt[t];
   if (!S.active) return;
@@ -831,6 +839,7 @@ __global__ void k_fin_alpha(CGState* stt, const int* slot_begin, const int* slot
 __global__ void k_fin_beta(CGState* stt, const int* slot_begin, const int* slot_end,
                            const int* zb, const int* ze, const double* part_upd, const double* part_rz,
                            int ncells, int jacobi) {
+  griddep_sync();
   FIN_PROLOGUE
   CGState S = stt[t];
   if (!S.active) return;
@@ -882,6 +891,7 @@ __global__ void k_restrict(const CellDesc* fine, const CellDesc* coarse, const N
                            const TF* __restrict__ rf, TCo* __restrict__ bc, TCo* __restrict__ xc,
                            const float* __restrict__ invdc, double omega, const CGState* stt, long long ntf,
                            long long ntc, const float* __restrict__ binvc) {
+  griddep_sync();
   const NodeUnit u = units[blockIdx.x];
   const int rhs = blockIdx.y;
   const CellDesc cc = coarse[u.cell], cf = fine[cc.parent];
@@ -937,6 +947,7 @@ template <typename TF, typename TCo>
 __global__ void k_prolong_add(const CellDesc* __restrict__ fine, const CellDesc* __restrict__ coarse,
                               const NodeUnit* __restrict__ units, TF* __restrict__ xf,
                               const TCo* __restrict__ ec, const CGState* stt, long long ntf, long long ntc) {
+  griddep_sync();
   const NodeUnit u = units[blockIdx.x];
   const int rhs = blockIdx.y;
   const CellDesc cf = fine[u.cell], cc = coarse[fine[u.cell].child];
@@ -1175,6 +1186,7 @@ template <typename TB, typename TX>
 __global__ void k_coarse_solve(const CellDesc* cells, const int* list, const double* Ainv,
                                const long long* aoff, const TB* b, TX* x, const CGState* stt,
                                long long ntot) {
+  griddep_sync();
   const int cell = list[blockIdx.x], rhs = blockIdx.y;
   const CellDesc cd = cells[cell];
   if (stt && !stt[cd.id * kNumRhs + rhs].active) return;
@@ -1478,6 +1490,7 @@ __global__ void k_dc_accum(const CellDesc* cells, const NodeUnit* units, double*
 template <typename TA, typename TB2>
 __global__ void k_dot(const CellDesc* cells, const NodeUnit* units, const TA* __restrict__ a, const TB2* __restrict__ b,
                       const CGState* stt, double* __restrict__ part, long long ntot) {
+  griddep_sync();
   const NodeUnit u = units[blockIdx.x];
   const int rhs = blockIdx.y;
   const CellDesc cd = cells[u.cell];
@@ -1524,6 +1537,7 @@ __global__ void k_norm2(const CellDesc* cells, const NodeUnit* units, const TV* 
 // the iterations run in this solve, so the loop always ends.
 __global__ void k_while_cond(cudaGraphConditionalHandle h, const CGState* __restrict__ stt, int ncells,
                              int listed, int* loop, int chunk, int limit) {
+  griddep_sync();
   __shared__ int alive;
   if (threadIdx.x == 0) alive = 0;
   __syncthreads();

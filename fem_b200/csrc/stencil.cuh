@@ -141,6 +141,7 @@ __device__ __forceinline__ void had_block(T (&w)[3][8], const HadK& K, T s) {
 template <typename T, int NT, int OUT, int NZ, typename TIn, typename TOut, typename TB, typename TC>
 __global__ void __launch_bounds__(NT, 1)
 stencil_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
+  griddep_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const StencilUnit un = a.units[blockIdx.x];
   const int rhs = blockIdx.y;
@@ -353,6 +354,7 @@ namespace femh {
 template <typename T, int NT, int OUT, int NZ, typename TIn, typename TOut, typename TB, typename TC>
 __global__ void __launch_bounds__(NT, 1)
 stencil2_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
+  griddep_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const StencilUnit un = a.units[blockIdx.x];
   const int rhs = blockIdx.y;
@@ -707,6 +709,7 @@ __device__ __forceinline__ void had_block_p(f2 (&w)[3][8], const HadK& K, float 
 template <int NT, int OUT, int NZ, typename TIn, typename TOut, typename TB, typename TC>
 __global__ void __launch_bounds__(NT, 1)
 stencilp_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
+  griddep_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const StencilUnit un = a.units[blockIdx.x];
   const int pr = blockIdx.y;   // load cases 2pr, 2pr+1
@@ -985,6 +988,7 @@ stencilp_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
 template <int NT, int OUT, int NZ, typename TIn, typename TOut, typename TB, typename TC>
 __global__ void __launch_bounds__(NT, 1)
 stencil2p_kernel(StencilArgs<TIn, TOut, TB, TC> a) {
+  griddep_sync();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const StencilUnit un = a.units[blockIdx.x];
   const int rhs = blockIdx.y;
@@ -1345,6 +1349,7 @@ __device__ __forceinline__ int bulk_rows(int idx, const int (&n)[NA], int& row) 
 template <int NT, int OUT, int NZ>
 __global__ void __launch_bounds__(NT, 1)
 stencil2b_kernel(StencilArgs<float, float, float, float> a) {
+  griddep_sync();
   static_assert(NZ > 0 && NZ % 4 == 0 && NT % NZ == 0, "staged rows need a compile-time pitch, multiple of 4");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int rhs = blockIdx.y;
@@ -1729,6 +1734,7 @@ __device__ __forceinline__ void had4s_inv(T (&v)[4]) {
 template <int NT, int OUT, int NZ, typename TIn>
 __global__ void __launch_bounds__(NT, 1)
 stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
+  griddep_sync();
   static_assert(NZ > 0 && NZ % 4 == 0 && NT % NZ == 0, "staged rows need a compile-time pitch, multiple of 4");
   constexpr int R = NT / NZ, NRU = R + 1, NRK = R, RB = R - 1;
   constexpr int bU = 0, bK = bU + 3 * NRU * NZ * (int)sizeof(TIn), bB = bK + NRK * NZ * 8,

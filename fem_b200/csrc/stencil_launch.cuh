@@ -17,8 +17,7 @@ void stencil_go(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, T
         CK(cudaFuncSetAttribute(fn3, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         attr3 = true;
       }
-      fn3<<<dim3(grid.x, kNumRhs / 2), NT, smem, H->stream>>>(a);
-      LAUNCH_CHECK(H);
+      launch(H, fn3, dim3(grid.x, kNumRhs / 2), NT, smem, a);
       return;
     }
   }
@@ -28,8 +27,7 @@ void stencil_go(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, T
       CK(cudaFuncSetAttribute(fn2, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       attr2 = true;
     }
-    fn2<<<grid, NT, smem, H->stream>>>(a);
-    LAUNCH_CHECK(H);
+    launch(H, fn2, grid, NT, smem, a);
     return;
   }
   bool& attr = attr1;
@@ -38,8 +36,7 @@ void stencil_go(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, T
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr = true;
   }
-  fn<<<grid, NT, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
+  launch(H, fn, grid, NT, smem, a);
 }
 
 // Two voxel rows per thread in packed FP32x2 lanes (variant 4).
@@ -51,8 +48,7 @@ void stencil_go4(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, 
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr = true;
   }
-  fn<<<grid, NT, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
+  launch(H, fn, grid, NT, smem, a);
 }
 
 // Two voxel rows per thread in packed FP32x2 lanes, inputs staged by bulk copies (variant 5).
@@ -64,8 +60,7 @@ void stencil_go5(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<float
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr = true;
   }
-  fn<<<grid, NT, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
+  launch(H, fn, grid, NT, smem, a);
 }
 
 // FP64 operator, one voxel row per thread, inputs staged by bulk copies (variant 6).
@@ -77,8 +72,7 @@ void stencil_go6(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, 
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     attr = true;
   }
-  fn<<<grid, NT, smem, H->stream>>>(a);
-  LAUNCH_CHECK(H);
+  launch(H, fn, grid, NT, smem, a);
 }
 
 // T = arithmetic type; in/out/b storage types as given.

@@ -98,6 +98,7 @@ __device__ __forceinline__ void tail_jacobi(const TailLevel& L, long long off, i
 
 template <typename T, typename TC>
 __global__ void __launch_bounds__(kTailThreads, 1) k_tail(const __grid_constant__ TailArgs a) {
+  griddep_sync();
   extern __shared__ __align__(16) unsigned char tail_smem[];
   const int rhs = blockIdx.y, tid = threadIdx.x;
   CellDesc cd[kTailLevels];
