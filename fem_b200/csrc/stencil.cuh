@@ -1723,6 +1723,24 @@ __device__ __forceinline__ void had4s_inv(T (&v)[4]) {
   v[0] = a0 - a1; v[1] = a0 + a1; v[2] = a2 - a3; v[3] = a2 + a3;
 }
 
+// Bytes of one stage of stencil1b_kernel, with the node-block inverses staged
+// (24 B per owned node) or the point ones (4 B), and of its whole CTA.
+constexpr int stage1b_bytes(int NT, int nz, int in_size, bool blocks) {
+  const int R = NT / nz;
+  return (3 * (R + 1) * nz * in_size + R * nz * 8 + 3 * (R - 1) * nz * 8 + (R - 1) * nz * (blocks ? 24 : 4) + 15) & ~15;
+}
+constexpr int stage1b_cta_bytes(int NT, int nz, int in_size, bool blocks) {
+  return kBulkSlots * stage1b_bytes(NT, nz, in_size, blocks) + 8 * 2 * (NT / nz) * 9 * nz + 8 * kBulkSlots + 64 * 8;
+}
+// Node-block sweeps stage the inverses wherever the CTA stays within 227 KB
+// (pitches 24 and from 48 up).  Read from global memory at the gather, their
+// latency stood in every step: 128^3 FP64 sweep 452 -> 379 us, 192^3 2.14 -> 1.50 ms,
+// 48^3 40 -> 35 us.
+constexpr bool stage1b_blocks(int NT, int nz, int in_size, int out) {
+  return (out == OUT_JACOBI || out == OUT_JACOBI_DOT) &&
+         stage1b_cta_bytes(NT, nz, in_size, true) + 64 <= 227 * 1024;
+}
+
 // FP64 operator, one voxel row per thread, inputs staged by bulk copies.
 // Schedule and staging of stencil2b_kernel (stage g = step g-1; u of node
 // plane ie+1, kc of voxel plane ie, b / invd of node plane ie-1), the
@@ -1730,7 +1748,9 @@ __device__ __forceinline__ void had4s_inv(T (&v)[4]) {
 // contributions half transformed (as in stencilp_kernel), arithmetic in FP64.
 // Thread (r, z) streams voxel (i, j0-1+r, z); row 0 is the y halo.  Stage
 // layout: U[3][R+1][NZ] (TIn), KC[R][NZ], B[3][R-1][NZ] (double), ID[R-1][NZ]
-// (float); Q[2][R][3 corners][3][NZ] doubles.  NZ is the row pitch, as there.
+// (float, or the node's 6 block inverses in a node-block sweep where they fit:
+// stage1b_blocks); Q[2][R][3 corners][3][NZ] doubles.  NZ is the row pitch, as
+// there.
 template <int NT, int OUT, int NZ, typename TIn>
 __global__ void __launch_bounds__(NT, 1)
 stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
@@ -1739,7 +1759,8 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
   constexpr int R = NT / NZ, NRU = R + 1, NRK = R, RB = R - 1;
   constexpr int bU = 0, bK = bU + 3 * NRU * NZ * (int)sizeof(TIn), bB = bK + NRK * NZ * 8,
                 bI = bB + 3 * RB * NZ * 8;
-  constexpr int SSB = (bI + RB * NZ * 4 + 15) & ~15;   // bytes per stage
+  constexpr bool BS = stage1b_blocks(NT, NZ, (int)sizeof(TIn), OUT);
+  constexpr int SSB = stage1b_bytes(NT, NZ, (int)sizeof(TIn), BS);   // bytes per stage
   constexpr int QS = R * 9 * NZ;                       // doubles per Q buffer
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const StencilUnit un = a.units[blockIdx.x];
@@ -1774,7 +1795,9 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
   const char* src_base = nullptr;
   int plane_lag = 0, src_off = 0, dst_off = 0, bytes = 0, esz = 0;
   unsigned tx_total = 0;
-  const bool ids = (OUT == OUT_JACOBI || OUT == OUT_JACOBI_DOT) && !a.binv;
+  const bool ids = (OUT == OUT_JACOBI || OUT == OUT_JACOBI_DOT) && (BS || !a.binv);
+  const int esI = BS && a.binv ? 24 : 4;   // bytes per node of the inverse diagonals
+  const float* src_I = esI == 24 ? a.binv + 6 * cd.off : a.invd + cd.off;
   constexpr int esU = (int)sizeof(TIn);
   if (nz == NZ) {
     if (tid < 32) {
@@ -1803,7 +1826,7 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
       if (OUT >= OUT_JACOBI) {
         for (int c = 0; c < 3; ++c)
           seg(a.b + ((long long)rhs * 3 + c) * st + cd.off, 8, -1, un.j0, rows, bB + c * RB * NZ * 8);
-        if (ids) seg(a.invd + cd.off, 4, -1, un.j0, rows, bI);
+        if (ids) seg(src_I, esI, -1, un.j0, rows, bI);
       }
     }
   } else {
@@ -1816,15 +1839,15 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
       src_base = k8 < 3    ? reinterpret_cast<const char*>(a.u + ((long long)rhs * 3 + c) * st + cd.off)
                  : k8 == 3 ? reinterpret_cast<const char*>(a.kc + cd.off)
                  : k8 < 7  ? reinterpret_cast<const char*>(a.b + ((long long)rhs * 3 + c) * st + cd.off)
-                           : reinterpret_cast<const char*>(a.invd + cd.off);
-      esz = k8 < 3 ? esU : k8 < 7 ? 8 : 4;
+                           : reinterpret_cast<const char*>(src_I);
+      esz = k8 < 3 ? esU : k8 < 7 ? 8 : esI;
       plane_lag = k8 < 3 ? 1 : k8 == 3 ? 0 : -1;
       src_off = wrapy(un.j0 - (k8 < 4 ? 1 : 0) + row) * nz;
       dst_off = k8 < 3 ? bU + (c * NRU + row) * NZ * esU : k8 == 3 ? bK + row * NZ * 8
-                : k8 < 7 ? bB + (c * RB + row) * NZ * 8 : bI + row * NZ * 4;
+                : k8 < 7 ? bB + (c * RB + row) * NZ * 8 : bI + row * NZ * esI;
       bytes = nz * esz;
     }
-    tx_total = (unsigned)nz * (unsigned)(esU * (n[0] + n[1] + n[2]) + 8 * (n[3] + n[4] + n[5] + n[6]) + 4 * n[7]);
+    tx_total = (unsigned)nz * (unsigned)(esU * (n[0] + n[1] + n[2]) + 8 * (n[3] + n[4] + n[5] + n[6]) + esI * n[7]);
   }
   const bool issuer = tid == 0 || bytes > 0;
   int pl_next = ((un.i0 - 2 + plane_lag) % nx + nx) % nx;
@@ -1899,8 +1922,9 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
       double dv[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) dv[c] = Bs[c * RB * NZ + rb] - y[c];
-      if (a.binv) {   // node-block sweep: the node's block inverse, read where the gather needs it
-        jacobi_dir<double>(a.binv, cd.off + pg + col, 0.0, dv);
+      if (a.binv) {   // node-block sweep: the node's block inverse, staged, or read where the gather needs it
+        if (BS) jacobi_dir<double>(Is, rb, 0.0, dv);
+        else jacobi_dir<double>(a.binv, cd.off + pg + col, 0.0, dv);
 #pragma unroll
         for (int c = 0; c < 3; ++c) dv[c] *= a.omega;
       } else {
@@ -1989,15 +2013,6 @@ stencil1b_kernel(StencilArgs<TIn, double, double, double> a) {
     block_reduce<1>(v, red);
     if (tid == 0) a.partials[(long long)un.slot * kNumRhs + rhs] = v[0];
   }
-}
-
-// Shared memory bytes of one stencil1b_kernel CTA.
-inline size_t stencil1b_smem_bytes(int NT, int nz, int in_size) {
-  const int R = NT / nz;
-  const size_t stage = ((size_t)3 * (R + 1) * nz * in_size + (size_t)R * nz * 8 + (size_t)3 * (R - 1) * nz * 8 +
-                        (size_t)(R - 1) * nz * 4 + 15) & ~(size_t)15;
-  return kBulkSlots * stage + sizeof(double) * 2 * (size_t)R * 9 * nz + sizeof(unsigned long long) * kBulkSlots +
-         64 * sizeof(double);
 }
 
 // Shared memory bytes of one stencil2b_kernel CTA (tiles of up to 2*TR-1 rows).

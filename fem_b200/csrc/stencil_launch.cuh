@@ -65,11 +65,12 @@ void stencil_go5(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<float
 
 // FP64 operator, one voxel row per thread, inputs staged by bulk copies (variant 6).
 template <int NT, int OUT, int NZ, typename TIn>
-void stencil_go6(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, double, double, double>& a) {
+void stencil_go6(femh_handle* H, dim3 grid, const StencilArgs<TIn, double, double, double>& a) {
+  constexpr int smem = stage1b_cta_bytes(NT, NZ, (int)sizeof(TIn), stage1b_blocks(NT, NZ, (int)sizeof(TIn), OUT));
   static bool attr = false;
   auto fn = stencil1b_kernel<NT, OUT, NZ, TIn>;
-  if (!attr) {   // (a few bytes of static shared memory come on top)
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+  if (!attr) {
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr = true;
   }
   launch(H, fn, grid, NT, smem, a);
@@ -168,17 +169,16 @@ void stencil(femh_handle* H, Level& L, bool smooth_only, const TIn* in, TOut* ou
                   (std::is_same<TIn, double>::value || std::is_same<TIn, float>::value)) {
       if (variant == 6) {
         const int c = stage_class(nz_spec > 0 ? nz_spec : maxnz);
-        const size_t sm6 = stencil1b_smem_bytes(stage_nt64(c), c, (int)sizeof(TIn));
         switch (c) {
-          case 16: stencil_go6<stage_nt64(16), OUT, 16>(H, grid, sm6, a); return;
-          case 24: stencil_go6<stage_nt64(24), OUT, 24>(H, grid, sm6, a); return;
-          case 32: stencil_go6<stage_nt64(32), OUT, 32>(H, grid, sm6, a); return;
-          case 48: stencil_go6<stage_nt64(48), OUT, 48>(H, grid, sm6, a); return;
-          case 64: stencil_go6<stage_nt64(64), OUT, 64>(H, grid, sm6, a); return;
-          case 96: stencil_go6<stage_nt64(96), OUT, 96>(H, grid, sm6, a); return;
-          case 128: stencil_go6<stage_nt64(128), OUT, 128>(H, grid, sm6, a); return;
-          case 192: stencil_go6<stage_nt64(192), OUT, 192>(H, grid, sm6, a); return;
-          case 256: stencil_go6<stage_nt64(256), OUT, 256>(H, grid, sm6, a); return;
+          case 16: stencil_go6<stage_nt64(16), OUT, 16>(H, grid, a); return;
+          case 24: stencil_go6<stage_nt64(24), OUT, 24>(H, grid, a); return;
+          case 32: stencil_go6<stage_nt64(32), OUT, 32>(H, grid, a); return;
+          case 48: stencil_go6<stage_nt64(48), OUT, 48>(H, grid, a); return;
+          case 64: stencil_go6<stage_nt64(64), OUT, 64>(H, grid, a); return;
+          case 96: stencil_go6<stage_nt64(96), OUT, 96>(H, grid, a); return;
+          case 128: stencil_go6<stage_nt64(128), OUT, 128>(H, grid, a); return;
+          case 192: stencil_go6<stage_nt64(192), OUT, 192>(H, grid, a); return;
+          case 256: stencil_go6<stage_nt64(256), OUT, 256>(H, grid, a); return;
           default: throw FemhError{FEMH_E_ARG, "staged FP64 stencil on an ineligible level"};
         }
       }
