@@ -1254,14 +1254,16 @@ struct Prec {
 // resolves ~1e-4 in angle, an FP64 one ~1e-6 is still meaningful).
 template <typename TM> constexpr double block_drop() { return sizeof(TM) == 8 ? 1e-12 : 1e-8; }
 
-// Partials of a 6x6 product A^T B of each cell's block: the upper triangle
-// (SYM) or all 36 entries, per node slot, into `part`.
-template <bool SYM, typename TA, typename TB>
-void block_gram(femh_handle* H, const char* name, const TA* a, const TB* b, double* part) {
+// Partials of the 6x6 product A^T B of each cell's block per node sub-slot into
+// part_ab, and with c != nullptr of C^T A into part_ca.
+template <typename TA, typename TB>
+void block_gram(femh_handle* H, const char* name, const TA* a, const TB* b, double* part_ab, const TB* c = nullptr,
+                double* part_ca = nullptr) {
   Level& L0 = H->levels[0];
   const dim3 grid((unsigned)(L0.all.nu.size() * H->bsub_g));
-  Prof prof_(H, name, 18.0 * (sizeof(TA) + sizeof(TB)) * (double)L0.ntot);
-  launch(H, k_bgram<SYM, TA, TB>, grid, 256, 0, L0.d_cells, L0.all.d_nu, a, b, H->d_bcg, part, L0.ntot, H->bsub_g);
+  Prof prof_(H, name, 18.0 * (sizeof(TA) + (c ? 2 : 1) * sizeof(TB)) * (double)L0.ntot);
+  launch(H, c ? k_bgram<true, TA, TB, TB> : k_bgram<false, TA, TB, TB>, grid, 256, 0, L0.d_cells, L0.all.d_nu, a, b, c,
+         H->d_bcg, part_ab, part_ca, L0.ntot, H->bsub_g);
 }
 
 // One block PCG iteration of the multigrid PCG (all live cells).
@@ -1285,7 +1287,7 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
   double* part_a = H->d_part_g;                                        // [Gram sub-slots][36]
   double* part_b = H->d_part_g + H->part_g_slots * nsub_g * 36;        // [Gram sub-slots][36]
   stencil<TV, OUT_APPLY_DOT>(H, L0, false, (const TP*)p, q, (const TV*)nullptr, kcg, H->d_part_s, stt, 0.0);
-  block_gram<true, TP, TV>(H, "k_bgram_pq", (const TP*)p, (const TV*)q, part_a);
+  block_gram<TP, TV>(H, "k_bgram_pq", (const TP*)p, (const TV*)q, part_a);
   {
     Prof prof_(H, "k_bfin_alpha", 0.0);
     launch(H, k_bfin_alpha, nc, 1024, 0, H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, part_a, nc, block_drop<TM>(), nsub_g);
@@ -1299,8 +1301,7 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
            H->d_bcg, H->d_part_b, L0.ntot, L0.binv, nsub);
   }
   TM* z = vcycle_of<TM, TMC>(H, r, rm, nullptr);
-  block_gram<false, TM, TV>(H, "k_bgram_zr", (const TM*)z, (const TV*)r, part_a);
-  block_gram<false, TV, TM>(H, "k_bgram_qz", (const TV*)q, (const TM*)z, part_b);
+  block_gram<TM, TV>(H, "k_bgram_z", (const TM*)z, (const TV*)r, part_a, (const TV*)q, part_b);
   {
     Prof prof_(H, "k_bfin_beta", 0.0);
     launch(H, k_bfin_beta, nc, 1024, 0, H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_b, part_a, part_b, nc,
@@ -1425,7 +1426,7 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
         LAUNCH_CHECK(H);
       }
       TM* z = vcycle_of<TM, TMC>(H, r, rm, nullptr);
-      block_gram<false, TM, TV>(H, "k_bgram_zr", (const TM*)z, (const TV*)r, H->d_part_g);
+      block_gram<TM, TV>(H, "k_bgram_z", (const TM*)z, (const TV*)r, H->d_part_g);
       {
         Prof prof_(H, "k_bfin_rz", 0.0);
         k_bfin_rz<<<nc, 1024, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_g, nc, H->bsub_g);

@@ -373,9 +373,6 @@ struct BlockCG {
 // iterations has stalled: its cell is solved again one load case at a time.
 constexpr int kBlockStallWindow = 200;
 
-// Index of (i, j), i <= j, in the 21 upper-triangle entries of a 6x6 matrix.
-__host__ __device__ constexpr int sym6(int i, int j) { return i * 6 - i * (i - 1) / 2 + (j - i); }
-
 // G X = s B (6x6, row-major, shared memory) by Cholesky on the columns in mask,
 // a column with a pivot below drop times its diagonal dropped (its row of X is
 // 0).  Returns false if a pivot is below -1e-8 times its diagonal (G indefinite
@@ -442,46 +439,98 @@ __device__ __forceinline__ SubUnit sub_unit(const NodeUnit* units, int S) {
   return r;
 }
 
-// Partials of the 6x6 matrix A^T B of one cell's block per sub-slot: its
-// upper triangle (SYM, 21 values) or all 36 entries a_i . b_j (i * 6 + j);
-// columns outside the block's mask read as 0.
-template <bool SYM, typename TA, typename TB>
-__global__ void __launch_bounds__(256, 2)
+// D += A B on the FP64 tensor cores: A 16 x 8 (lane l holds rows l / 4 and + 8
+// of columns l % 4 and + 4), B 8 x 8 (rows l % 4 and + 4, column l / 4), D 16 x 8
+// (rows l / 4 and + 8, columns 2 (l % 4) and the next).  Lane l's values of load
+// case l / 4 at two nodes serve as rows of A or as columns of B.
+__device__ __forceinline__ void dmma1688(double (&d)[4], double lo0, double hi0, double lo1, double hi1, double b0,
+                                         double b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(lo0), "d"(hi0), "d"(lo1), "d"(hi1), "d"(b0), "d"(b1));
+}
+__device__ __forceinline__ void ld_pair(const double* p, bool vec, bool in0, bool in1, double (&v)[2]) {
+  if (vec && in0 && in1) {
+    const double2 t = __ldg(reinterpret_cast<const double2*>(p));
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+    v[0] = in0 ? __ldg(p) : 0.0;
+    v[1] = in1 ? __ldg(p + 1) : 0.0;
+  }
+}
+__device__ __forceinline__ void ld_pair(const float* p, bool vec, bool in0, bool in1, double (&v)[2]) {
+  if (vec && in0 && in1) {
+    const float2 t = __ldg(reinterpret_cast<const float2*>(p));
+    v[0] = (double)t.x;
+    v[1] = (double)t.y;
+  } else {
+    v[0] = in0 ? (double)__ldg(p) : 0.0;
+    v[1] = in1 ? (double)__ldg(p + 1) : 0.0;
+  }
+}
+__device__ __forceinline__ void ld_pair(const __nv_bfloat16* p, bool, bool in0, bool in1, double (&v)[2]) {
+  v[0] = in0 ? (double)ld_val(p) : 0.0;
+  v[1] = in1 ? (double)ld_val(p + 1) : 0.0;
+}
+
+// Partials of the 6x6 matrix A^T B (entry i * 6 + j = a_i . b_j) of one cell's
+// block per sub-slot, and with TWO of C^T A as well, A read once; columns
+// outside the block's mask read as 0.  A warp takes eight nodes at a time, lane
+// l the nodes 2 (l % 4) and the next of load case l / 4, and sums the products
+// on the FP64 tensor cores: four registers for both matrices, where a thread
+// per node needed 36 accumulators each (72 spilled) and their reduction over
+// the CTA.  Z^T R and (K P)^T Z: 128^3 two passes of 125 + 121 us -> one of 215
+// (0.52 of measured HBM), 64^3 31 + 29 -> 36; P^T K P 119 -> 113 and 21 -> 17
+// (0.82).  Four nodes a lane, four times fewer or more CTAs and 8 x 8 x 4
+// products all measured the same within 5%.
+template <bool TWO, typename TA, typename TB, typename TC>
+__global__ void __launch_bounds__(256)
 k_bgram(const CellDesc* cells, const NodeUnit* units, const TA* __restrict__ a, const TB* __restrict__ b,
-        const BlockCG* bst, double* __restrict__ part, long long ntot, int nsub) {
+        const TC* __restrict__ c, const BlockCG* bst, double* __restrict__ part_ab, double* __restrict__ part_ca,
+        long long ntot, int nsub) {
   griddep_sync();
-  constexpr int NV = SYM ? 21 : 36;
   const SubUnit su = sub_unit(units, nsub);
   const CellDesc cd = cells[su.u.cell];
   const int mask = bst[cd.id].live ? bst[cd.id].mask : 0;
-  double v[NV];
+  if (!mask) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int i = lane >> 2, q = lane & 3;
+  const bool on = i < kNumRhs && (mask >> i & 1);
+  // pairs start at even level nodes; with an odd plane stride pairs are loaded one by one
+  const bool vec = (ntot & 1) == 0;
+  const long long begin = cd.off + su.begin, end = cd.off + su.end;
+  double d[4] = {0.0, 0.0, 0.0, 0.0};   // rows 0-7: b_i . a_j, rows 8-15: c_i . a_j
+  for (long long g0 = (begin & ~1LL) + 8 * warp; g0 < end; g0 += 8 * nw) {
+    const long long g = g0 + 2 * q;
+    const bool in0 = on && g >= begin && g < end, in1 = on && g + 1 >= begin && g + 1 < end;
+    double av[3][2], bv[3][2], cv[3][2];
 #pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = 0.0;
-  if (mask) {
-    for (long long n = su.begin + threadIdx.x; n < su.end; n += blockDim.x) {
-      const long long g = cd.off + n;
-#pragma unroll 1
-      for (int c = 0; c < 3; ++c) {
-        double av[6], bv[6];
+    for (int k = 0; k < 3; ++k) {
+      const long long o = ((long long)i * 3 + k) * ntot + g;
+      ld_pair(a + o, vec, in0, in1, av[k]);
+      ld_pair(b + o, vec, in0, in1, bv[k]);
+      if (TWO) ld_pair(c + o, vec, in0, in1, cv[k]);
+    }
 #pragma unroll
-        for (int j = 0; j < 6; ++j) {
-          const long long o = ((long long)j * 3 + c) * ntot + g;
-          const bool in = mask >> j & 1;
-          av[j] = in ? (double)ld_val(a + o) : 0.0;
-          bv[j] = in ? (double)ld_val(b + o) : 0.0;
-        }
+    for (int k = 0; k < 3; ++k)
+      dmma1688(d, bv[k][0], TWO ? cv[k][0] : 0.0, bv[k][1], TWO ? cv[k][1] : 0.0, av[k][0], av[k][1]);
+  }
+  __shared__ double red[TWO ? 2 : 1][8][36];   // per warp
+  if (i < kNumRhs && q < 3) {
 #pragma unroll
-        for (int i = 0; i < 6; ++i)
-#pragma unroll
-          for (int j = SYM ? i : 0; j < 6; ++j) v[SYM ? sym6(i, j) : i * 6 + j] += av[i] * bv[j];
-      }
+    for (int h = 0; h < 2; ++h) {
+      red[0][warp][(2 * q + h) * 6 + i] = d[h];
+      if (TWO) red[TWO ? 1 : 0][warp][i * 6 + 2 * q + h] = d[2 + h];
     }
   }
-  __shared__ double red[32 * NV];
-  block_reduce<NV>(v, red);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) part[su.sub * NV + k] = v[k];
+  __syncthreads();
+  if (threadIdx.x < (TWO ? 72 : 36)) {
+    const int m = threadIdx.x / 36, k = threadIdx.x % 36;
+    double v = 0.0;
+    for (int w = 0; w < nw; ++w) v += red[m][w][k];
+    (m ? part_ca : part_ab)[su.sub * 36 + k] = v;
+  }
 }
 
 // Sums of a cell's per-slot partials by a 1024-thread CTA in a fixed order
@@ -572,12 +621,12 @@ __global__ void __launch_bounds__(1024) k_bfin_alpha(BlockCG* bst, CGState* stt,
   const int cell = blockIdx.x, lane = threadIdx.x;
   BlockCG& B = bst[cell];
   if (!B.live) return;
-  __shared__ double red[1024], g[21], G[36], A[36], ZR[36];
-  cta_sums<1, 21>({part_g}, {21}, {sb[cell] * nsub}, {se[cell] * nsub}, red, g);
+  __shared__ double red[1024], g[36], G[36], A[36], ZR[36];
+  cta_sums<1, 36>({part_g}, {36}, {sb[cell] * nsub}, {se[cell] * nsub}, red, g);
   if (lane >= 32) return;
   for (int k = lane; k < 36; k += 32) {
     const int i = k / 6, j = k % 6;
-    G[k] = g[i <= j ? sym6(i, j) : sym6(j, i)];
+    G[k] = i <= j ? g[k] : g[j * 6 + i];   // symmetric to the last bit
     ZR[k] = B.zr[k];
   }
   __syncwarp();
