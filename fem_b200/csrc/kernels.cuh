@@ -1130,9 +1130,9 @@ __global__ void __launch_bounds__(96) k_coarse_assemble(const CellDesc* cells, c
 // ran on one CTA per cell, a chain of m pivots each with a pass over the
 // trailing matrix: 1.60 ms at m = 192, 26.3 ms at 315, 150 ms at 600.  Here a
 // step is one launch whose CTAs (one per lower-triangle tile and cell) each
-// invert the 32 x 32 pivot block themselves (32 short pivots in shared memory,
+// invert the 32 x 32 pivot block themselves (32 short pivots in registers,
 // the same pivots as Cholesky's) and do the rank-32 update of their tile, so
-// the chain is ceil(m / 32) launches.  Steps go from one buffer to the other:
+// the chain is ceil(m / 32) launches of ~16 us.  Steps go from one buffer to the other:
 // tiles read the pivot row and column of the previous step while the same
 // launch rewrites them.  Tiles i > j are stored twice, so the inverse is
 // symmetric to the last bit, which the V-cycle needs to be a symmetric
@@ -1158,62 +1158,64 @@ __global__ void __launch_bounds__(256) k_coarse_sweep(const CellDesc* cells, con
     const int gi = bi * kSweep + r, gj = bj * kSweep + x;
     return gi < m && gj < m ? src[(long long)gi * m + gj] : (bi == bj && r == x ? 1.0 : 0.0);
   };
-  double a[4];
+  double a[4], v[4];
+  __shared__ double prow[2][kSweep], pcol[2][kSweep];   // pivot row and column, of this pivot and the next
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int r = y + 8 * q;
-    D[r][x] = at(step, step, r);
+    v[q] = at(step, step, r);
     P[r][x] = at(ti, step, r);      // A_ik
     Q[r][x] = at(tj, step, r);      // A_jk = A_kj^T
     a[q] = at(ti, tj, r);
+    if (r == 0) prow[0][x] = v[q];
+    if (x == 0) pcol[0][r] = v[q];
   }
-  // D <- A_kk^-1: scalar sweeps, one pivot at a time, in place
+  // v <- -A_kk^-1: scalar sweeps, one pivot at a time, in registers; a barrier
+  // per pivot passes the next pivot's row and column on
   for (int p = 0; p < kSweep; ++p) {
     __syncthreads();
-    double d = D[p][p];
-    d = 1.0 / (d > 0.0 ? d : 1e-300);
-    const double cx = D[p][x];
-    double v[4];
+    const double* row = prow[p & 1];
+    const double* col = pcol[p & 1];
+    const double piv = row[p], cx = row[x];
+    const double d = 1.0 / (piv > 0.0 ? piv : 1e-300);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int r = y + 8 * q;
-      const double cr = D[r][p];
-      v[q] = r == p ? (x == p ? -d : cx * d) : (x == p ? cr * d : D[r][x] - cr * d * cx);
+      const double cr = col[r];
+      v[q] = r == p ? (x == p ? -d : cx * d) : (x == p ? cr * d : v[q] - cr * d * cx);
+      if (r == p + 1) prow[(p + 1) & 1][x] = v[q];
+      if (x == p + 1) pcol[(p + 1) & 1][r] = v[q];
     }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) D[y + 8 * q][x] = v[q];
   }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) D[y + 8 * q][x] = v[q];
   __syncthreads();
   // U = A_ik D (D holds -A_kk^-1)
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int r = y + 8 * q;
-    double u = 0.0;
+  double u[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 8
-    for (int p = 0; p < kSweep; ++p) u -= P[r][p] * D[p][x];
-    U[r][x] = u;
+  for (int p = 0; p < kSweep; ++p) {
+    const double dx = D[p][x];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) u[q] -= P[y + 8 * q][p] * dx;
   }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) U[y + 8 * q][x] = u[q];
   __syncthreads();
-  double v[4];
+  const bool krow = ti == step && tj != step;   // tile of the pivot row: (A_jk D)^T
+#pragma unroll
+  for (int q = 0; q < 4; ++q) a[q] = krow ? 0.0 : a[q];
+#pragma unroll 8
+  for (int p = 0; p < kSweep; ++p) {
+    const double qx = Q[x][p];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a[q] -= (krow ? D[p][y + 8 * q] : U[y + 8 * q][p]) * qx;
+  }
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int r = y + 8 * q;
-    if (ti == step && tj == step) {
-      v[q] = r >= x ? D[r][x] : D[x][r];   // -D
-    } else if (tj == step) {
-      v[q] = U[r][x];                      // A_ik D
-    } else if (ti == step) {               // (A_jk D)^T: row r of the pivot block, column x of tile j
-      double u = 0.0;
-#pragma unroll 8
-      for (int p = 0; p < kSweep; ++p) u -= Q[x][p] * D[p][r];
-      v[q] = u;
-    } else {
-      double u = a[q];
-#pragma unroll 8
-      for (int p = 0; p < kSweep; ++p) u -= U[r][p] * Q[x][p];
-      v[q] = u;
-    }
+    if (ti == step && tj == step) v[q] = r >= x ? D[r][x] : D[x][r];   // -D
+    else if (tj == step) v[q] = u[q];                                  // A_ik D
+    else v[q] = a[q];
     if (step == T - 1) v[q] = -v[q];
   }
   __syncthreads();   // P is free: the tile on its way to the mirrored store
