@@ -535,32 +535,43 @@ k_bgram(const CellDesc* cells, const NodeUnit* units, const TA* __restrict__ a, 
 
 // Sums of a cell's per-slot partials by a 1024-thread CTA in a fixed order
 // (deterministic): value v of set q (NQ sets of n[q] values, slots [b[q], e[q])
-// of part[q]) is added up by G thread groups, group g over the slots b + g,
+// of part[q]) is added up by G[q] threads, thread g over the slots b + g,
 // b + g + G, ... (coalesced rows, eight loads in flight per thread), then the G
-// group sums by one thread.  out[v] (shared memory, the sets one after another)
-// is valid after the call in every thread.  256 threads without the unrolling
-// took 24 us of a 128^3 iteration for the three sums of the beta step.
-template <int NQ, int NV>
-__device__ __forceinline__ void cta_sums(const double* const (&part)[NQ], const int (&n)[NQ], const int (&b)[NQ],
-                                         const int (&e)[NQ], double* red, double* out) {
-  constexpr int G = 1024 / NV;
-  const int t = threadIdx.x, v = t % NV, g = t / NV;
-  if (g < G) {
-    int q = 0, w = v;
-    while (q + 1 < NQ && w >= n[q]) w -= n[q++];
-    const double* p = part[q] + w;
-    const int nq = n[q], end = e[q];
-    double acc = 0.0;
+// sums by one thread.  sum n[q] G[q] <= 1024.  out (shared memory, the sets one
+// after another) is valid after the call in every thread.  256 threads without
+// the unrolling took 24 us of a 128^3 iteration for the three sums of the beta
+// step; with the same G for its sets the 4096 slots of ||r||^2 took 25.
+template <int NQ>
+__device__ __forceinline__ void cta_sums(const double* const (&part)[NQ], const int (&n)[NQ], const int (&G)[NQ],
+                                         const int (&b)[NQ], const int (&e)[NQ], double* red, double* out) {
+  const int t = threadIdx.x;
+  int first = 0, val = 0;   // threads and values of the sets before
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int nq = n[q], Gq = G[q], u = t - first;
+    if (u >= 0 && u < nq * Gq) {
+      const double* p = part[q] + u % nq;
+      const int end = e[q];
+      double acc = 0.0;
 #pragma unroll 8
-    for (int sl = b[q] + g; sl < end; sl += G) acc += p[(long long)sl * nq];
-    red[g * NV + v] = acc;
+      for (int sl = b[q] + u / nq; sl < end; sl += Gq) acc += p[(long long)sl * nq];
+      red[t] = acc;
+    }
+    first += nq * Gq;
   }
   __syncthreads();
-  if (t < NV) {
-    double acc = 0.0;
+  first = 0;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int nq = n[q], Gq = G[q], v = t - val;
+    if (v >= 0 && v < nq) {
+      double acc = 0.0;
 #pragma unroll 8
-    for (int g2 = 0; g2 < G; ++g2) acc += red[g2 * NV + t];
-    out[t] = acc;
+      for (int g = 0; g < Gq; ++g) acc += red[first + g * nq + v];
+      out[t] = acc;
+    }
+    first += nq * Gq;
+    val += nq;
   }
   __syncthreads();
 }
@@ -608,7 +619,7 @@ __global__ void __launch_bounds__(1024) k_bfin_rz(BlockCG* bst, CGState* stt, co
   BlockCG& B = bst[cell];
   if (!B.live) return;
   __shared__ double red[1024], Z[36];
-  cta_sums<1, 36>({part_zr}, {36}, {sb[cell] * nsub}, {se[cell] * nsub}, red, Z);
+  cta_sums<1>({part_zr}, {36}, {28}, {sb[cell] * nsub}, {se[cell] * nsub}, red, Z);
   if (lane >= 32) return;
   if (!zr_positive(Z, B.mask)) return block_stop(B, stt, cell, B.mask, CG_BLOCK_FAIL);
   for (int k = lane; k < 36; k += 32) B.zr[k] = Z[k];
@@ -622,7 +633,7 @@ __global__ void __launch_bounds__(1024) k_bfin_alpha(BlockCG* bst, CGState* stt,
   BlockCG& B = bst[cell];
   if (!B.live) return;
   __shared__ double red[1024], g[36], G[36], A[36], ZR[36];
-  cta_sums<1, 36>({part_g}, {36}, {sb[cell] * nsub}, {se[cell] * nsub}, red, g);
+  cta_sums<1>({part_g}, {36}, {28}, {sb[cell] * nsub}, {se[cell] * nsub}, red, g);
   if (lane >= 32) return;
   for (int k = lane; k < 36; k += 32) {
     const int i = k / 6, j = k % 6;
@@ -650,8 +661,8 @@ __global__ void __launch_bounds__(1024) k_bfin_beta(BlockCG* bst, CGState* stt, 
   if (!B.live) return;
   const int b = sb[cell], e = se[cell];
   __shared__ double red[1024], sums[78], T[36], G[36];
-  cta_sums<3, 78>({part_zr, part_qz, part_upd}, {36, 36, kNumRhs}, {b * nsub_g, b * nsub_g, b * nsub},
-                  {e * nsub_g, e * nsub_g, e * nsub}, red, sums);
+  cta_sums<3>({part_zr, part_qz, part_upd}, {36, 36, kNumRhs}, {10, 10, 50}, {b * nsub_g, b * nsub_g, b * nsub},
+              {e * nsub_g, e * nsub_g, e * nsub}, red, sums);
   if (lane >= 32) return;
   const double *Z = sums, *Q = sums + 36, *rr = sums + 72;
   const unsigned full = 0xffffffffu;
