@@ -1264,8 +1264,12 @@ void block_gram(femh_handle* H, const char* name, const TA* a, const TB* b, doub
   Level& L0 = H->levels[0];
   const dim3 grid((unsigned)(L0.all.nu.size() * H->bsub_g));
   Prof prof_(H, name, 18.0 * (sizeof(TA) + (c ? 2 : 1) * sizeof(TB)) * (double)L0.ntot);
-  launch(H, c ? k_bgram<true, TA, TB, TB> : k_bgram<false, TA, TB, TB>, grid, 256, 0, L0.d_cells, L0.all.d_nu, a, b, c,
-         H->d_bcg, part_ab, part_ca, L0.ntot, H->bsub_g);
+  // The single product's registers would let five CTAs onto a multiprocessor;
+  // with four the 1024 CTAs of 128^3 make two even waves (144 -> 116 us), so it
+  // asks for shared memory that holds it to four.
+  const size_t four = c ? 0 : 45 * 1024;
+  launch(H, c ? k_bgram<true, TA, TB, TB> : k_bgram<false, TA, TB, TB>, grid, 256, four, L0.d_cells, L0.all.d_nu, a, b,
+         c, H->d_bcg, part_ab, part_ca, L0.ntot, H->bsub_g);
 }
 
 // One block PCG iteration of the multigrid PCG (all live cells).

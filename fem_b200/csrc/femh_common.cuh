@@ -86,10 +86,39 @@ enum CGStatus : int { CG_RUNNING = 0, CG_CONVERGED = 1, CG_MAXITER = 2, CG_BREAK
 
 template <typename T> struct VT { using type = T; };
 
-__device__ __forceinline__ double ld_val(const double* p) { return __ldg(p); }
-__device__ __forceinline__ float ld_val(const float* p) { return __ldg(p); }
+// Loads of vectors that the loop's kernels write: coherent loads after
+// griddep_sync().  A kernel of the loop is resident while the kernel before it
+// still writes, so the read-only path (__ldg, ld.global.nc), whose data must
+// not change while the kernel runs, is not open to them; nor may they be plain
+// reads of `const T* __restrict__` parameters, which the compiler turns into
+// that path.  `volatile` keeps them after the wait; they carry no "memory"
+// clobber, so other work moves around them (no kernel reads back what it wrote).
+__device__ __forceinline__ double ld_val(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ float ld_val(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
 __device__ __forceinline__ float ld_val(const __nv_bfloat16* p) {
-  return __bfloat162float(*p);
+  unsigned short v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(__cvta_generic_to_global(p)));
+  return __bfloat162float(__ushort_as_bfloat16(v));
+}
+template <typename T> using LdT = decltype(ld_val((const T*)nullptr));   // what ld_val returns for a T
+// Two values from a pair-aligned address.
+__device__ __forceinline__ double2 ld_val2(const double* p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ float2 ld_val2(const float* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(__cvta_generic_to_global(p)));
+  return v;
 }
 __device__ __forceinline__ void st_val(double* p, double v) { *p = v; }
 __device__ __forceinline__ void st_val(float* p, float v) { *p = v; }
@@ -122,7 +151,8 @@ __device__ __forceinline__ void jacobi_dir(const float* __restrict__ binv, long 
 // dependents (launch() in state.cuh), so a launch overlaps its predecessor's
 // run instead of following its end.  No kernel of the loop may return or touch
 // memory before this call: completion of one must imply completion of all
-// before it.
+// before it.  After it, what the loop writes is read with coherent loads
+// (ld_val, or plain reads through pointers that are not __restrict__).
 __device__ __forceinline__ void griddep_sync() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

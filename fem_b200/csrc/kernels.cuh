@@ -263,10 +263,11 @@ __global__ void k_cg_init(const CellDesc* cells, const NodeUnit* units, const TB
 // when rm != nullptr, r in the V-cycle's storage type (the level-0 right-hand
 // side its sweeps read).
 template <typename TV, typename TP, typename TQ, typename TZ>
-__global__ void k_cg_update(const CellDesc* cells, const NodeUnit* units, TV* __restrict__ x, TV* __restrict__ r, const TP* __restrict__ p,
-                            const TQ* __restrict__ q, const float* __restrict__ invd, TZ* __restrict__ z0,
-                            TZ* __restrict__ rm, double omega, const CGState* stt,
-                            double* __restrict__ part, long long ntot, const float* __restrict__ binv) {
+__global__ void __launch_bounds__(256, 2)
+k_cg_update(const CellDesc* cells, const NodeUnit* units, TV* __restrict__ x, TV* __restrict__ r,
+            const TP* __restrict__ p, const TQ* __restrict__ q, const float* __restrict__ invd, TZ* __restrict__ z0,
+            TZ* __restrict__ rm, double omega, const CGState* stt, double* __restrict__ part, long long ntot,
+            const float* __restrict__ binv) {
   griddep_sync();
   const NodeUnit u = units[blockIdx.x];
   const int rhs = blockIdx.y;
@@ -275,29 +276,59 @@ __global__ void k_cg_update(const CellDesc* cells, const NodeUnit* units, TV* __
   double v[2] = {0.0, 0.0};
   if (S.active) {
     const double al = S.alpha;
-    #pragma unroll 4
-  for (long long n = u.begin + threadIdx.x; n < u.end; n += blockDim.x) {
-      const long long g = cd.off + n;
-      const double id = (double)invd[g];
-      double rvs[3];
+    // A thread issues the loads of U nodes before its first store, which later
+    // loads cannot pass.  The stores' addresses are formed anew: kept from the
+    // loads they would take as many registers as the values.  FP64 with U = 4
+    // spills at the 128 registers that two CTAs leave (33 x 45 x 37, a whole
+    // Jacobi iteration: U = 1 39.9, 2 39.6, 4 41.8 us).
+    constexpr int U = sizeof(TV) == 8 ? 2 : 4;
+    const long long base = (long long)rhs * 3 * ntot + cd.off;
+    const unsigned end = (unsigned)u.end, bd = blockDim.x;
+#pragma unroll 1
+    for (unsigned n0 = (unsigned)u.begin + threadIdx.x; n0 < end; n0 += U * bd) {
+      LdT<TV> xs[U][3], rs[U][3];
+      LdT<TP> ps[U][3];
+      LdT<TQ> qs[U][3];
+      float ids[U];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const long long o = ((long long)rhs * 3 + c) * ntot + g;
-        const double pv = (double)ld_val(p + o);
-        const double xv = (double)ld_val(x + o) + al * pv;
-        const double rv = (double)ld_val(r + o) - al * (double)ld_val(q + o);
-        st_val(x + o, xv);
-        st_val(r + o, rv);
-        v[0] += rv * rv;
-        v[1] += rv * id * rv;
-        if (z0 && !binv) st_val(z0 + o, omega * id * rv);
-        if (rm) st_val(rm + o, rv);
-        rvs[c] = rv;
+      for (int k = 0; k < U; ++k) {
+        const unsigned n = n0 + k * bd;
+        if (n >= end) break;
+        ids[k] = invd[cd.off + n];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const long long o = base + c * ntot;
+          ps[k][c] = ld_val(p + o + n);
+          xs[k][c] = ld_val(x + o + n);
+          rs[k][c] = ld_val(r + o + n);
+          qs[k][c] = ld_val(q + o + n);
+        }
       }
-      if (z0 && binv) {   // node-block Jacobi: z0 = omega B r
-        jacobi_dir<double>(binv, g, 0.0, rvs);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) st_val(z0 + ((long long)rhs * 3 + c) * ntot + g, omega * rvs[c]);
+      for (int k = 0; k < U; ++k) {
+        unsigned n = n0 + k * bd;
+        if (n >= end) break;
+        asm volatile("" : "+r"(n));
+        const double id = (double)ids[k];
+        double rvs[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const long long o = base + c * ntot;
+          const double xv = (double)xs[k][c] + al * (double)ps[k][c];
+          const double rv = (double)rs[k][c] - al * (double)qs[k][c];
+          st_val(x + o + n, xv);
+          st_val(r + o + n, rv);
+          v[0] += rv * rv;
+          v[1] += rv * id * rv;
+          if (z0 && !binv) st_val(z0 + o + n, omega * id * rv);
+          if (rm) st_val(rm + o + n, rv);
+          rvs[c] = rv;
+        }
+        if (z0 && binv) {   // node-block Jacobi: z0 = omega B r
+          jacobi_dir<double>(binv, cd.off + n, 0.0, rvs);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) st_val(z0 + base + c * ntot + n, omega * rvs[c]);
+        }
       }
     }
   }
@@ -320,14 +351,35 @@ __global__ void k_cg_dir(const CellDesc* cells, const NodeUnit* units, TP* __res
   const CGState S = stt[cd.id * kNumRhs + rhs];
   if (!S.active) return;
   const double be = S.beta;
-  #pragma unroll 4
-  for (long long n = u.begin + threadIdx.x; n < u.end; n += blockDim.x) {
-    const long long g = cd.off + n;
+  const bool mg = zvec && !S.fallback;
+  constexpr int U = 4;   // as in k_cg_update
+  const long long base = (long long)rhs * 3 * ntot + cd.off;
+  const unsigned end = (unsigned)u.end, bd = blockDim.x;
+#pragma unroll 1
+  for (unsigned n0 = (unsigned)u.begin + threadIdx.x; n0 < end; n0 += U * bd) {
+    double zs[U][3];
+    LdT<TP> ps[U][3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const long long o = ((long long)rhs * 3 + c) * ntot + g;
-      const double z = (zvec && !S.fallback) ? (double)ld_val(zvec + o) : (double)invd[g] * (double)ld_val(r + o);
-      st_val(p + o, be == 0.0 ? z : z + be * (double)ld_val(p + o));
+    for (int k = 0; k < U; ++k) {
+      const unsigned n = n0 + k * bd;
+      if (n >= end) break;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const long long o = base + c * ntot;
+        zs[k][c] = mg ? (double)ld_val(zvec + o + n) : (double)invd[cd.off + n] * (double)ld_val(r + o + n);
+        ps[k][c] = ld_val(p + o + n);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      unsigned n = n0 + k * bd;
+      if (n >= end) break;
+      asm volatile("" : "+r"(n));
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double z = zs[k][c];
+        st_val(p + base + c * ntot + n, be == 0.0 ? z : z + be * (double)ps[k][c]);
+      }
     }
   }
 }
@@ -449,24 +501,15 @@ __device__ __forceinline__ void dmma1688(double (&d)[4], double lo0, double hi0,
       : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
       : "d"(lo0), "d"(hi0), "d"(lo1), "d"(hi1), "d"(b0), "d"(b1));
 }
-__device__ __forceinline__ void ld_pair(const double* p, bool vec, bool in0, bool in1, double (&v)[2]) {
+template <typename T>
+__device__ __forceinline__ void ld_pair(const T* p, bool vec, bool in0, bool in1, double (&v)[2]) {
   if (vec && in0 && in1) {
-    const double2 t = __ldg(reinterpret_cast<const double2*>(p));
-    v[0] = t.x;
-    v[1] = t.y;
-  } else {
-    v[0] = in0 ? __ldg(p) : 0.0;
-    v[1] = in1 ? __ldg(p + 1) : 0.0;
-  }
-}
-__device__ __forceinline__ void ld_pair(const float* p, bool vec, bool in0, bool in1, double (&v)[2]) {
-  if (vec && in0 && in1) {
-    const float2 t = __ldg(reinterpret_cast<const float2*>(p));
+    const auto t = ld_val2(p);
     v[0] = (double)t.x;
     v[1] = (double)t.y;
   } else {
-    v[0] = in0 ? (double)__ldg(p) : 0.0;
-    v[1] = in1 ? (double)__ldg(p + 1) : 0.0;
+    v[0] = in0 ? (double)ld_val(p) : 0.0;
+    v[1] = in1 ? (double)ld_val(p + 1) : 0.0;
   }
 }
 __device__ __forceinline__ void ld_pair(const __nv_bfloat16* p, bool, bool in0, bool in1, double (&v)[2]) {
@@ -1042,11 +1085,18 @@ __global__ void k_prolong_add(const CellDesc* __restrict__ fine, const CellDesc*
         }
       }
     }
+    const bool two = n + 1 < u.end;
+    TF* px = xf + (long long)rhs * 3 * ntf + cf.off + n;
+    LdT<TF> x0[3], x1[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {   // all before the first store
+      x0[c] = ld_val(px + c * ntf);
+      x1[c] = two ? ld_val(px + c * ntf + 1) : (LdT<TF>)0;
+    }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      TF* px = xf + ((long long)rhs * 3 + c) * ntf + cf.off + n;
-      st_val(px, (double)ld_val(px) + a0[c]);
-      if (n + 1 < u.end) st_val(px + 1, (double)ld_val(px + 1) + a1[c]);
+      st_val(px + c * ntf, (double)x0[c] + a0[c]);
+      if (two) st_val(px + c * ntf + 1, (double)x1[c] + a1[c]);
     }
   }
 }
@@ -1597,7 +1647,7 @@ __global__ void k_norm2(const CellDesc* cells, const NodeUnit* units, const TV* 
 // more than half of the `listed` cells still iterate (otherwise the host
 // compacts the unit lists to the live cells and relaunches).  loop[0] counts
 // the iterations run in this solve, so the loop always ends.
-__global__ void k_while_cond(cudaGraphConditionalHandle h, const CGState* __restrict__ stt, int ncells,
+__global__ void k_while_cond(cudaGraphConditionalHandle h, const CGState* stt, int ncells,
                              int listed, int* loop, int chunk, int limit) {
   griddep_sync();
   __shared__ int alive;

@@ -75,16 +75,19 @@ __device__ __forceinline__ void tail_apply(const T* __restrict__ x, T* __restric
   }
 }
 
-// b - K x at one node from the corner contributions.
+// b - K x at one node from the corner contributions (b: shared memory or the
+// loop's global vector, so not __restrict__).
 template <typename T>
-__device__ __forceinline__ void tail_residual(const T* __restrict__ F, const T* __restrict__ b, long long bs, int n,
-                                              int q, T (&d)[3]) {
+__device__ __forceinline__ void tail_residual(const T* __restrict__ F, const T* b, long long bs, int n, int q,
+                                              T (&d)[3]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) d[c] = b[c * bs + q];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     T y = (T)0;
 #pragma unroll
     for (int a = 0; a < 8; ++a) y += F[(3 * a + c) * n + q];
-    d[c] = b[c * bs + q] - y;
+    d[c] -= y;
   }
 }
 
