@@ -462,6 +462,7 @@ bool block_pcg(const femh_config& c) {
   return c.block_cg && c.solver == FEMH_GMG_PCG && (c.precision == FEMH_FP64 || c.precision == FEMH_MIXED_PC);
 }
 
+constexpr int kMaxCoarseNodes = 1536;   // of the dense coarse solve
 std::vector<int> level_dims(const femh_config& c, int nx, int ny, int nz) {
   std::vector<int> d = {nx, ny, nz};
   if (c.solver != FEMH_GMG_PCG) return d;
@@ -470,7 +471,7 @@ std::vector<int> level_dims(const femh_config& c, int nx, int ny, int nz) {
     nx /= 2; ny /= 2; nz /= 2;
     d.insert(d.end(), {nx, ny, nz});
   }
-  if ((long long)nx * ny * nz * 3 > 3 * 1536)
+  if ((long long)nx * ny * nz > kMaxCoarseNodes)
     throw FemhError{FEMH_E_ARG, "multigrid needs cells that halve down to <= 1536 coarse nodes; use Jacobi-PCG"};
   return d;
 }
@@ -1053,9 +1054,11 @@ void prepare_operator(femh_handle* H) {
       {
         Prof prof_(H, "k_coarse_assemble", 0.0);
         auto fn = k_coarse_assemble<TC>;
-        const size_t sm = sizeof(double) * 3 * L.coarse_maxm;   // up to 108 KB (1536 nodes)
-        if (sm > 48 * 1024)
-          CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        const size_t sm = sizeof(double) * 3 * L.coarse_maxm;
+        // the limit belongs to the function: always the largest level's, so that
+        // handles of other sizes in other threads cannot lower it before the launch
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(double) * 9 * kMaxCoarseNodes));
         fn<<<dim3(n, (unsigned)L.coarse_maxm / 3), 96, sm, s>>>(L.d_cells, L.d_coarse_list, (const TC*)L.kc, H->d_K0,
                                                                L.d_A, L.d_Awork, L.d_aoff);
         LAUNCH_CHECK(H);
