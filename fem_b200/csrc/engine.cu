@@ -494,7 +494,7 @@ double cell_setup_bytes(const femh_config& c, int nx, int ny, int nz) {
     if (gmg && c.block_jacobi) b += n * 24.0;              // node-block inverses
     if (l > 0 || gmg) b += n * 36.0 * msz;                 // xa, xb
     if (l > 0) b += n * 18.0 * msz;                        // bv
-    if (gmg && l == nl - 1) b += 2.0 * (3.0 * n) * (3.0 * n) * 8.0;   // coarse A, Awork
+    if (gmg && l == nl - 1) b += 2.0 * (3.0 * n) * (3.0 * n) * 8.0 + n * 8.0;   // coarse A, Awork, Adiag
   }
   const double nv = (double)nx * ny * nz;
   b += nv * (3 * 8.0 + 18 * 8.0 * 2);                      // rho_in, rho_used, kc64, b64, x64
@@ -693,6 +693,7 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
       CK(cudaStreamSynchronize(s));   // local vectors go out of scope
       L.d_A = ar.arr<double>(o);
       L.d_Awork = ar.arr<double>(o);
+      L.d_Adiag = ar.arr<double>(L.ntot);
     }
   }
   H->tail = gmg ? tail_level(H, msz) : nlev;
@@ -1060,13 +1061,13 @@ void prepare_operator(femh_handle* H) {
         CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(double) * 9 * kMaxCoarseNodes));
         fn<<<dim3(n, (unsigned)L.coarse_maxm / 3), 96, sm, s>>>(L.d_cells, L.d_coarse_list, (const TC*)L.kc, H->d_K0,
-                                                               L.d_A, L.d_Awork, L.d_aoff);
+                                                               L.d_A, L.d_Awork, L.d_aoff, L.d_Adiag);
         LAUNCH_CHECK(H);
       }
       for (int step = 0; step < T; ++step) {
         Prof prof_(H, "k_coarse_sweep", 0.0);
         k_coarse_sweep<<<dim3(n, (unsigned)(T * (T + 1) / 2)), 256, 0, s>>>(L.d_cells, L.d_coarse_list, L.d_A,
-                                                                           L.d_Awork, L.d_aoff, step);
+                                                                           L.d_Awork, L.d_aoff, L.d_Adiag, step);
         LAUNCH_CHECK(H);
       }
     }

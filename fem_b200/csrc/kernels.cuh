@@ -1134,37 +1134,68 @@ __global__ void k_jacobi0(const CellDesc* cells, const NodeUnit* units, const TB
 }
 
 // Dense coarse operator, FP64: A = sum_e kc_e K0(1) scattered to the periodic
-// DOFs, plus the mean diagonal times the projector on the three translations,
-// A's null space (A + a e_c e_c^T / nodes for each component c): on a
-// right-hand side without net force the regular matrix's solution is A's, with
-// no net translation.  A is m x m, m = 3 * nodes.  One 96-thread CTA per (node, cell) owns the
-// node's three rows, gathers its 8 voxels (one after another: a corner pair of
-// two voxels may meet in the same entry) in shared memory and writes the rows
-// once.  A CTA per cell that scattered voxel after voxel took 66 us at 64
-// nodes and 162 us at 105; a row owner needs 8 steps whatever the size (~4 us).
+// DOFs, with the rows and columns of one node zero: the inversion leaves the
+// unknowns of zero pivots out, so that node stays put and the solution of a
+// right-hand side without net force is A's up to a translation, which no residual
+// sees.  It is the node with the largest diagonal (the first of them): it takes
+// up the net force that rounding leaves, and a node among soft voxels would yield
+// to it (40 iterations instead of 2 on a frame of 1 in 1e-9).  (The mean
+// diagonal times the projector on the translations, added to A instead, couples
+// every pair of nodes at the stiff voxels' scale: soft voxels lose their digits --
+// contrasts of 1e12 made the preconditioner indefinite -- and the unknowns of
+// voxels without stiffness no longer drop out.)  diag[node] is A's diagonal, the
+// same for the three components.  A is m x m, m = 3 * nodes.  One 96-thread CTA
+// per (node, cell) owns the node's three rows, gathers its 8 voxels (one after
+// another: a corner pair of two voxels may meet in the same entry) in shared
+// memory and writes the rows once.  A CTA per cell that scattered voxel after
+// voxel took 66 us at 64 nodes and 162 us at 105; a row owner needs 8 steps
+// whatever the size (~4 us).
 // Cells whose sweep takes an odd number of block steps start in `work`, so
 // that the last step of every cell writes A (k_coarse_sweep).
 constexpr int kSweep = 32;   // block size of the coarse inversion
 template <typename TC>
 __global__ void __launch_bounds__(96) k_coarse_assemble(const CellDesc* cells, const int* list, const TC* kc,
                                                         const double* K0, double* A, double* work,
-                                                        const long long* aoff) {
+                                                        const long long* aoff, double* diag) {
   extern __shared__ double rows[];   // [3][m]
   const CellDesc cd = cells[list[blockIdx.x]];
   const int nn = cd.nx * cd.ny * cd.nz, m = 3 * nn, n = blockIdx.y;
   if (n >= nn) return;
   double* M = ((m + kSweep - 1) / kSweep % 2 ? work : A) + aoff[blockIdx.x];
-  // mean diagonal: every voxel adds kc_e K0[0] to each of its 8 corners' diagonals
-  // (every CTA adds the same voxels in the same order)
-  double sum[1] = {0.0};
-  for (int e = threadIdx.x; e < nn; e += blockDim.x) sum[0] += (double)kc[cd.off + e];
-  __shared__ double red[32];
-  __shared__ double shift;
-  block_reduce<1>(sum, red);
-  if (threadIdx.x == 0) shift = 8.0 * K0[0] * sum[0] / ((double)nn * (double)nn);
+  // the fixed node (every CTA of the cell finds the same one)
+  double mx = -1.0;
+  int pin = 0;
+  for (int q = threadIdx.x; q < nn; q += blockDim.x) {
+    int i, j, k;
+    node_ijk(q, cd.ny, cd.nz, i, j, k);
+    double s = 0.0;
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+      s += (double)kc[cd.off + lin(wrap(i - (a >> 2 & 1), cd.nx), wrap(j - (a >> 1 & 1), cd.ny),
+                                   wrap(k - (a & 1), cd.nz), cd.ny, cd.nz)];
+    if (s > mx) {
+      mx = s;
+      pin = q;
+    }
+  }
+  auto take = [&](double v, int q) {   // the larger one, the first of equals
+    if (v > mx || (v == mx && q < pin)) {
+      mx = v;
+      pin = q;
+    }
+  };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    take(__shfl_xor_sync(0xffffffffu, mx, o), __shfl_xor_sync(0xffffffffu, pin, o));
+  __shared__ double best[3];
+  __shared__ int node[3];
+  if (threadIdx.x % 32 == 0) {
+    best[threadIdx.x / 32] = mx;
+    node[threadIdx.x / 32] = pin;
+  }
+  for (int t = threadIdx.x; t < 3 * m; t += blockDim.x) rows[t] = 0.0;
   __syncthreads();
-  for (int t = threadIdx.x; t < 3 * m; t += blockDim.x) rows[t] = t / m == t % m % 3 ? shift : 0.0;
-  __syncthreads();
+  for (int w = 0; w < 3; ++w) take(best[w], node[w]);
   int i, j, k;
   node_ijk(n, cd.ny, cd.nz, i, j, k);
   const int t = threadIdx.x, aq = t / 9, cp = t / 3 % 3, cq = t % 3;   // 72 of the threads: corner, row, column
@@ -1179,7 +1210,9 @@ __global__ void __launch_bounds__(96) k_coarse_assemble(const CellDesc* cells, c
     }
     __syncthreads();
   }
-  for (int q = t; q < 3 * m; q += blockDim.x) M[(long long)3 * n * m + q] = rows[q];
+  if (t == 0) diag[cd.off + n] = n == pin ? 0.0 : rows[3 * n];
+  for (int q = t; q < 3 * m; q += blockDim.x)
+    M[(long long)3 * n * m + q] = n == pin || q % m / 3 == pin ? 0.0 : rows[q];
 }
 
 // Explicit inverse of every cell's SPD coarse matrix by symmetric block sweeps
@@ -1197,10 +1230,13 @@ __global__ void __launch_bounds__(96) k_coarse_assemble(const CellDesc* cells, c
 // tiles read the pivot row and column of the previous step while the same
 // launch rewrites them.  Tiles i > j are stored twice, so the inverse is
 // symmetric to the last bit, which the V-cycle needs to be a symmetric
-// preconditioner.  A pivot that is not positive (a floating part of a
-// zero-stiffness cell) is replaced by 1e-300.
+// preconditioner.  A pivot that is zero up to rounding -- not above kPivotFloor
+// times A's diagonal there: the fixed node, voxels without stiffness, parts held by
+// nothing else -- leaves its unknown out: its row and column of the inverse are
+// zero.
+constexpr double kPivotFloor = 32 * 1.1102230246251565e-16;
 __global__ void __launch_bounds__(256) k_coarse_sweep(const CellDesc* cells, const int* list, double* A, double* work,
-                                                      const long long* aoff, int step) {
+                                                      const long long* aoff, const double* diag, int step) {
   const CellDesc cd = cells[list[blockIdx.x]];
   const int m = 3 * cd.nx * cd.ny * cd.nz, T = (m + kSweep - 1) / kSweep;
   if (step >= T) return;
@@ -1221,6 +1257,9 @@ __global__ void __launch_bounds__(256) k_coarse_sweep(const CellDesc* cells, con
   };
   double a[4], v[4];
   __shared__ double prow[2][kSweep], pcol[2][kSweep];   // pivot row and column, of this pivot and the next
+  __shared__ double least[kSweep];   // pivots up to here are zero
+  const int gp = step * kSweep + x;
+  const double dg = y == 0 && gp < m ? diag[cd.off + gp / 3] : 0.0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int r = y + 8 * q;
@@ -1231,6 +1270,7 @@ __global__ void __launch_bounds__(256) k_coarse_sweep(const CellDesc* cells, con
     if (r == 0) prow[0][x] = v[q];
     if (x == 0) pcol[0][r] = v[q];
   }
+  if (y == 0) least[x] = kPivotFloor * dg;
   // v <- -A_kk^-1: scalar sweeps, one pivot at a time, in registers; a barrier
   // per pivot passes the next pivot's row and column on
   for (int p = 0; p < kSweep; ++p) {
@@ -1238,7 +1278,7 @@ __global__ void __launch_bounds__(256) k_coarse_sweep(const CellDesc* cells, con
     const double* row = prow[p & 1];
     const double* col = pcol[p & 1];
     const double piv = row[p], cx = row[x];
-    const double d = 1.0 / (piv > 0.0 ? piv : 1e-300);
+    const double d = piv > least[p] ? 1.0 / piv : 0.0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int r = y + 8 * q;

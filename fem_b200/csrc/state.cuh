@@ -125,6 +125,7 @@ struct Level {
   long long* d_cell_aoff = nullptr;              // the same by cell (coarsest cells of this level)
   double* d_A = nullptr;
   double* d_Awork = nullptr;
+  double* d_Adiag = nullptr;                     // diagonal of the coarse matrices, by node of the level
   int coarse_maxm = 0;
   void* kc = nullptr;     // TC
   float* invd = nullptr;
