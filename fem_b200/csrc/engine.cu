@@ -541,10 +541,14 @@ void build_setup(femh_handle* H, const std::vector<int>& shapes, const std::vect
   if (H->shape_key == shapes && H->h_key == hs && H->prec_key == c.precision && H->solver_key == c.solver &&
       H->bf16_key == c.store_bf16)
     return;
+  // no set-up from here to the end: a call refused in between leaves no key for
+  // the next one to match
+  H->shape_key.clear();
   release_loops(H);
   H->setup.release();
   release_stage(H);
   H->levels.clear();
+  H->ncells = 0;
   H->solved = false;
   H->have_x = false;
   Arena& ar = H->setup;
