@@ -20,7 +20,7 @@ SOURCES = [os.path.join(CSRC, f) for f in (
     "engine.cu", "stencil_f32_sweep.cu", "stencil_f32_apply.cu", "stencil_f64_sweep.cu", "stencil_f64_apply.cu")] + [
     os.path.join(HERE, "host", "femh_host.cpp")]
 HEADERS = [os.path.join(CSRC, f) for f in (
-    "femh_common.cuh", "stencil.cuh", "stencil_launch.cuh", "kernels.cuh", "state.cuh", "tail.cuh")] + [
+    "femh_common.cuh", "stencil.cuh", "stencil_launch.cuh", "kernels.cuh", "state.cuh", "tail.cuh", "smem_limits.hpp")] + [
     os.path.join(HERE, "host", "femh_host.hpp")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 

@@ -1060,10 +1060,7 @@ void prepare_operator(femh_handle* H) {
         Prof prof_(H, "k_coarse_assemble", 0.0);
         auto fn = k_coarse_assemble<TC>;
         const size_t sm = sizeof(double) * 3 * L.coarse_maxm;
-        // the limit belongs to the function: always the largest level's, so that
-        // handles of other sizes in other threads cannot lower it before the launch
-        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(double) * 9 * kMaxCoarseNodes));
+        allow_smem(H, fn, (int)sizeof(double) * 9 * kMaxCoarseNodes);
         fn<<<dim3(n, (unsigned)L.coarse_maxm / 3), 96, sm, s>>>(L.d_cells, L.d_coarse_list, (const TC*)L.kc, H->d_K0,
                                                                L.d_A, L.d_Awork, L.d_aoff, L.d_Adiag);
         LAUNCH_CHECK(H);
@@ -1202,11 +1199,7 @@ void vcycle_tail(femh_handle* H, TM* x) {
   for (int q = 0; q < a.pre; ++q) a.w_pre[q] = H->w_pre[q];
   for (int q = 0; q < a.post; ++q) a.w_post[q] = H->w_post[q];
   auto fn = k_tail<TM, TMC>;
-  static bool attr = false;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
-    attr = true;
-  }
+  allow_smem(H, fn, kTailSmem);
   Prof prof_(H, "k_tail", 36.0 * sizeof(TM) * (double)T.ntot);
   launch(H, fn, dim3((unsigned)T.cells.size(), kNumRhs), kTailThreads, smem, a);
 }

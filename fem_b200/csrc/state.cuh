@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/femh.h"
+#include "smem_limits.hpp"
 #include "stencil.cuh"
 
 using namespace femh;
@@ -208,6 +209,7 @@ struct femh_handle {
   std::vector<double> C_last;
 
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  SmemLimits smem_limits;        // kernels whose shared memory limit this handle has raised
   int wait_limit = kWaitLimit;   // try_wait rounds of the staged kernels' stage waits
   int nsm = 1;                   // multiprocessors of the device (persistent stencil CTAs)
   // persistent stencil CTAs are split evenly over the six load cases; the inner
@@ -258,6 +260,14 @@ namespace femh_engine {
     if ((H)->capturing) (H)->cap_count++;        \
     else (H)->launches++;                        \
   } while (0)
+
+// Raises a kernel's dynamic shared memory limit to `bytes`, the most that any
+// of its launches takes (the same in every call, see smem_limits.hpp).
+template <typename... P>
+void allow_smem(femh_handle* H, void (*fn)(P...), int bytes) {
+  H->smem_limits.raise((const void*)fn,
+                       [&] { CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); });
+}
 
 // Launch of a kernel of the CG loop, as a programmatic dependent of the kernel
 // before it (griddep_sync()) while launches are a part of the time: 3 to 6% of

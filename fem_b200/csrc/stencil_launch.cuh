@@ -9,57 +9,38 @@ namespace femh_engine {
 
 template <typename T, int NT, int OUT, int NZ, typename TIn, typename TOut, typename TB, typename TC>
 void stencil_go(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, TOut, TB, TC>& a, int variant) {
-  static bool attr1 = false, attr2 = false, attr3 = false;
   if constexpr (std::is_same<T, float>::value) {
     if (variant == 3) {   // two load cases per CTA in packed FP32x2 lanes
       auto fn3 = stencilp_kernel<NT, OUT, NZ, TIn, TOut, TB, TC>;
-      if (!attr3) {
-        CK(cudaFuncSetAttribute(fn3, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        attr3 = true;
-      }
+      allow_smem(H, fn3, 227 * 1024);
       launch(H, fn3, dim3(grid.x, kNumRhs / 2), NT, smem, a);
       return;
     }
   }
   if (variant == 2) {
     auto fn2 = stencil2_kernel<T, NT, OUT, NZ, TIn, TOut, TB, TC>;
-    if (!attr2) {
-      CK(cudaFuncSetAttribute(fn2, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr2 = true;
-    }
+    allow_smem(H, fn2, 200 * 1024);
     launch(H, fn2, grid, NT, smem, a);
     return;
   }
-  bool& attr = attr1;
   auto fn = stencil_kernel<T, NT, OUT, NZ, TIn, TOut, TB, TC>;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
+  allow_smem(H, fn, 200 * 1024);
   launch(H, fn, grid, NT, smem, a);
 }
 
 // Two voxel rows per thread in packed FP32x2 lanes (variant 4).
 template <int NT, int OUT, int NZ, typename TIn, typename TOut, typename TB, typename TC>
 void stencil_go4(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<TIn, TOut, TB, TC>& a) {
-  static bool attr = false;
   auto fn = stencil2p_kernel<NT, OUT, NZ, TIn, TOut, TB, TC>;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
+  allow_smem(H, fn, 200 * 1024);
   launch(H, fn, grid, NT, smem, a);
 }
 
 // Two voxel rows per thread in packed FP32x2 lanes, inputs staged by bulk copies (variant 5).
 template <int NT, int OUT, int NZ>
 void stencil_go5(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<float, float, float, float>& a) {
-  static bool attr = false;
   auto fn = stencil2b_kernel<NT, OUT, NZ>;
-  if (!attr) {   // (a few bytes of static shared memory come on top)
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
+  allow_smem(H, fn, 200 * 1024);   // (a few bytes of static shared memory come on top)
   launch(H, fn, grid, NT, smem, a);
 }
 
@@ -67,12 +48,8 @@ void stencil_go5(femh_handle* H, dim3 grid, size_t smem, const StencilArgs<float
 template <int NT, int OUT, int NZ, typename TIn>
 void stencil_go6(femh_handle* H, dim3 grid, const StencilArgs<TIn, double, double, double>& a) {
   constexpr int smem = stage1b_cta_bytes(NT, NZ, (int)sizeof(TIn), stage1b_blocks(NT, NZ, (int)sizeof(TIn), OUT));
-  static bool attr = false;
   auto fn = stencil1b_kernel<NT, OUT, NZ, TIn>;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
+  allow_smem(H, fn, smem);
   launch(H, fn, grid, NT, smem, a);
 }
 
