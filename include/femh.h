@@ -82,7 +82,10 @@ typedef struct {
                              binary benchmark cells CG then stalls near 1e-4 (the rounded
                              search directions lose conjugacy): keep 0 there.  FEMH_MIXED_PC
                              with block_cg keeps its search directions in FP64 regardless */
-  int graph_chunk;        /* CG iterations per captured CUDA graph (0 = no graphs) */
+  int graph_chunk;        /* CG iterations per pass of the captured loop (0 = no graphs), an
+                             upper limit: FEMH_GMG_PCG runs at most 4 a pass, whose launches
+                             past convergence cost more than the pass.  Results do not
+                             depend on it */
   int coarse_avg;         /* coarse voxel modulus from its 8 children: 0 arithmetic mean
                              (rediscretisation of the mean), 1 geometric, 2 harmonic */
   int autotune;           /* 1: time the stencil's x-chunk length per level at set-up */
@@ -90,14 +93,16 @@ typedef struct {
                              thread, 2 two rows per thread, 3 two load cases per thread in
                              packed FP32x2 lanes, 4 two rows per thread in packed FP32x2
                              lanes, 5 as 4 with the inputs staged in shared memory by bulk
-                             copies (3-5: FP32 operators; FP64 ones use 1 or 2), 6 one row
-                             per thread in FP64 with staged inputs (FP64 operators; FP32
-                             ones use 1), 7 as 5 with one persistent CTA per multiprocessor
-                             running a balanced run of units (FP32 operators; levels of one
-                             z extent).  5-7 need every cell of a level to have a z extent
-                             in {16,24,32,48,64,128 (,256 for 6)} (levels of mixed extents
-                             launch one kernel per extent; 7 runs as 5 there); elsewhere 4
-                             and 1 run */
+                             copies, 6 one row per thread in FP64 with staged inputs, 7 as 5
+                             with one persistent CTA per multiprocessor running a balanced
+                             run of units (levels of one z extent; 5 elsewhere).  3, 4, 5
+                             and 7 are for FP32 operators; FP64 ones then use 1 (for 3) or
+                             2.  6 is for FP64 operators; FP32 ones then use 2.  Staging
+                             (5-7) takes levels of one z extent: 16, 24, 32, and every
+                             multiple of 4 from 36 to 192 (5, 7) or 256 (6); and levels of
+                             several extents that are all in {16,24,32,48,64,128,256}, one
+                             kernel per extent (5: up to 128).  Elsewhere 5 and 7 run as 4,
+                             6 as 2 */
   int warm_start;         /* 1: a solve on the same cells as the handle's previous solve
                              starts from that solution (chi) instead of zero -- the
                              line-search / descent case of fast_fem/run3d.cpp:238-289;
