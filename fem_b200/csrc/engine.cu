@@ -1250,6 +1250,7 @@ struct Prec {
   using K = TK;
   using M = TM;
   using MC = TMC;
+  static constexpr bool block = sizeof(TV) == 8 && sizeof(TP) == 8;   // block PCG (block_pcg) runs in it
 };
 
 // Block PCG: directions dropped from G = P^T K P below this pivot ratio
@@ -1324,7 +1325,9 @@ void pcg_iteration_block(femh_handle* H, const typename PR::K* kcg) {
 // One PCG iteration (all cells / load cases; inactive ones skip their work).
 template <class PR>
 void pcg_iteration(femh_handle* H, const typename PR::K* kcg, bool blk) {
-  if (blk) return pcg_iteration_block<PR>(H, kcg);
+  if constexpr (PR::block) {
+    if (blk) return pcg_iteration_block<PR>(H, kcg);
+  }
   using TV = typename PR::V;
   using TP = typename PR::P;
   using TM = typename PR::M;
@@ -1400,7 +1403,7 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
   TP* p = (TP*)H->cg_p;
   TM* rm = (gmg && sizeof(TM) != sizeof(TV)) ? (TM*)H->cg_rm : nullptr;
   CGState* stt = H->d_state;
-  const bool blk = block && block_pcg(c) && sizeof(TV) == 8 && sizeof(TP) == 8;
+  const bool blk = PR::block && block && block_pcg(c);
   for (auto& S : H->state) {
     S.tol = tol;
     S.max_iter = max_iter;
@@ -1426,24 +1429,26 @@ void pcg(femh_handle* H, const TB* b, const typename PR::K* kcg, int max_iter, d
                                                           L0.invd, H->w_pre[0], stt, L0.ntot, L0.binv);
       LAUNCH_CHECK(H);
     }
-    if (blk) {   // block PCG: Z^T R of the start, P = Z
-      {
-        Prof prof_(H, "k_binit", 0.0);
-        k_binit<<<cdiv(nc, 128), 128, 0, s>>>(H->d_bcg, stt, nc);
-        LAUNCH_CHECK(H);
-      }
-      TM* z = vcycle_of<TM, TMC>(H, r, rm, nullptr);
-      block_gram<TM, TV>(H, "k_bgram_z", (const TM*)z, (const TV*)r, H->d_part_g);
-      {
-        Prof prof_(H, "k_bfin_rz", 0.0);
-        k_bfin_rz<<<nc, 1024, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_g, nc, H->bsub_g);
-        LAUNCH_CHECK(H);
-      }
-      {
-        Prof prof_(H, "k_bdir", 0.0);
-        auto fn = H->bt == 64 ? k_bdir<64, TP, TM> : k_bdir<256, TP, TM>;
-        launch(H, fn, dim3((unsigned)(L0.all.nu.size() * H->bsub)), H->bt, 0, L0.d_cells, L0.all.d_nu, p,
-               (const TM*)z, H->d_bcg, L0.ntot, 1, H->bsub);
+    if constexpr (PR::block) {   // block PCG: Z^T R of the start, P = Z
+      if (blk) {
+        {
+          Prof prof_(H, "k_binit", 0.0);
+          k_binit<<<cdiv(nc, 128), 128, 0, s>>>(H->d_bcg, stt, nc);
+          LAUNCH_CHECK(H);
+        }
+        TM* z = vcycle_of<TM, TMC>(H, r, rm, nullptr);
+        block_gram<TM, TV>(H, "k_bgram_z", (const TM*)z, (const TV*)r, H->d_part_g);
+        {
+          Prof prof_(H, "k_bfin_rz", 0.0);
+          k_bfin_rz<<<nc, 1024, 0, s>>>(H->d_bcg, stt, L0.d_nu_sb, L0.d_nu_se, H->d_part_g, nc, H->bsub_g);
+          LAUNCH_CHECK(H);
+        }
+        {
+          Prof prof_(H, "k_bdir", 0.0);
+          auto fn = H->bt == 64 ? k_bdir<64, TP, TM> : k_bdir<256, TP, TM>;
+          launch(H, fn, dim3((unsigned)(L0.all.nu.size() * H->bsub)), H->bt, 0, L0.d_cells, L0.all.d_nu, p,
+                 (const TM*)z, H->d_bcg, L0.ntot, 1, H->bsub);
+        }
       }
     }
   }
@@ -2080,7 +2085,6 @@ femh_status femh_homogenize_batch(femh_handle* H, int ncell, const femh_cell* ce
     for (auto& I : infos)
       if (I.status != FEMH_OK) code = I.status;
     if (dLdC) {
-      Level& L0 = H->levels[0];
       std::vector<double> W(21 * ncell);
       for (int ci = 0; ci < ncell; ++ci) {
         int t = 0;
@@ -2104,7 +2108,6 @@ femh_status femh_homogenize_grad(femh_handle* H, const double dLdC[36], double* 
     if (!H->solved || H->ncells != 1) throw FemhError{FEMH_E_STATE, "call femh_homogenize first"};
     if (!dLdC || !dLdrho) throw FemhError{FEMH_E_ARG, "dLdC and dLdrho must not be NULL"};
     CK(cudaSetDevice(H->device));
-    Level& L0 = H->levels[0];
     double W[21];
     int t = 0;
     for (int I = 0; I < 6; ++I)
@@ -2157,7 +2160,6 @@ femh_status femh_field_gradient(femh_handle* H, const double dLdC[36], double dL
       H->fmap_key = key;
       H->fmap_nparam = nparam;
     }
-    Level& L0 = H->levels[0];
     double W[21];
     int t = 0;
     for (int I = 0; I < 6; ++I)
@@ -2209,7 +2211,6 @@ femh_status femh_dCdrho(femh_handle* H, double* out, int out_on_device) {
     if (!H->solved || H->ncells != 1) throw FemhError{FEMH_E_STATE, "call femh_homogenize first"};
     if (!out) throw FemhError{FEMH_E_ARG, "out must not be NULL"};
     CK(cudaSetDevice(H->device));
-    Level& L0 = H->levels[0];
     EnergyArgs a = energy_args(H, H->hk);
     a.out = out_on_device ? out : stage(H, 21 * (size_t)H->nvox);
     energy_launch<EN_DCDRHO>(H, a);

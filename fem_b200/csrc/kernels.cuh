@@ -512,10 +512,6 @@ __device__ __forceinline__ void ld_pair(const T* p, bool vec, bool in0, bool in1
     v[1] = in1 ? (double)ld_val(p + 1) : 0.0;
   }
 }
-__device__ __forceinline__ void ld_pair(const __nv_bfloat16* p, bool, bool in0, bool in1, double (&v)[2]) {
-  v[0] = in0 ? (double)ld_val(p) : 0.0;
-  v[1] = in1 ? (double)ld_val(p + 1) : 0.0;
-}
 
 // Partials of the 6x6 matrix A^T B (entry i * 6 + j = a_i . b_j) of one cell's
 // block per sub-slot, and with TWO of C^T A as well, A read once; columns
