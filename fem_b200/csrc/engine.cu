@@ -506,12 +506,18 @@ double cell_setup_bytes(const femh_config& c, int nx, int ny, int nz) {
 
 // First level of the V-cycle's fused end (tail.cuh): the finest level below 0
 // on which every cell's vectors fit one CTA's shared memory (12^3 nodes in
-// FP32, 10^3 in FP64), while its CTAs -- one per cell and load case, one per
-// multiprocessor -- stay within eight waves; beyond that the level kernels,
-// which spread a level over all multiprocessors, are the faster ones again.
+// FP32, 10^3 in FP64) and whose coarsest levels give each of the CTA's threads
+// one unknown at most: with more, the CTA passes over the dense inverse twice
+// where k_coarse_solve spreads it over 1024 threads.  Whole solves, level
+// kernels -> fused, by the nodes of the coarsest level: 125 (20^3) 3.2 -> 2.87
+// ms, 147 (28x28x12) 3.20 -> 3.04; 175 (20x20x28) 3.52 -> 3.62, 225 (20x20x36)
+// 3.94 -> 4.21, (40x40x72) 8.54 -> 9.79; FP64 125 and 147 even, 175 3.66 -> 3.86.
+// At most eight waves of its CTAs, one per cell and load case and one per
+// multiprocessor: a bound, not a crossing -- batches of 16^3 and 24^3 cells are
+// faster with it at every count measured (0.5 to 16 waves: 3 to 14%), 32^3 by 1%.
 // Per block iteration: 16^3 154 -> 126 us, 40x56x24 278 -> 273, 64^3 706 -> 684.
 constexpr int kTailSmem = 220 * 1024;
-constexpr int kTailCoarse = 256;   // coarsest nodes: beyond, one CTA's pass over the dense inverse is all there is
+constexpr int kTailCoarse = kTailThreads / 3;
 int tail_level(const femh_handle* H, size_t msz) {
   const int nlev = (int)H->levels.size();
   if (H->cfg.pre_smooth > 8 || H->cfg.post_smooth > 8) return nlev;

@@ -30,6 +30,16 @@ def test_fused_end_for_few_cells_level_kernels_for_many():
     assert "k_tail" not in _kernels(e, lambda: e.batch([rho] * many))
 
 
+@pytest.mark.parametrize("prec", [femh.FP64, femh.MIXED_PC])
+def test_fused_end_with_an_unknown_per_thread(prec):
+    """7 x 7 x 3 = 147 coarsest nodes, 441 unknowns for its 512 threads, and
+    5 x 5 x 7 = 175 nodes, 525 unknowns: two passes over the dense inverse."""
+    for shape, fused in [((28, 28, 12), True), ((20, 20, 28), False)]:
+        e = femh.Engine(precision=prec, autotune=0)
+        rho = np.random.default_rng(2).uniform(0.2, 1.0, shape)
+        assert ("k_tail" in _kernels(e, lambda: e.homogenize(rho))) == fused
+
+
 @pytest.mark.parametrize("kw", [dict(stencil_variant=5, precision=femh.MIXED_PC),
                                 dict(stencil_variant=6), dict(stencil_variant=7, precision=femh.MIXED)])
 def test_batch_on_one_z_extent_between_pitches(kw):
