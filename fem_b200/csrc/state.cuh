@@ -270,12 +270,19 @@ void allow_smem(femh_handle* H, void (*fn)(P...), int bytes) {
 }
 
 // Launch of a kernel of the CG loop, as a programmatic dependent of the kernel
-// before it (griddep_sync()) while launches are a part of the time: 3 to 6% of
-// an iteration up to 64^3 (Jacobi-PCG at 32^3 25.5 -> 24.6 us, 48^3 FP64 450 ->
-// 433, 64^3 539 -> 528).  With 2 M voxels the early CTAs only take slots from
-// kernels of several waves (128^3 FP64 4.59 -> 4.68 ms), so larger sets launch
-// plainly; griddep_sync() then returns at once.
-constexpr long long kEarlyLaunchVoxels = 1 << 20;
+// before it (griddep_sync()) while launches are a part of the time.  With more
+// voxels the early CTAs only take slots from kernels of several waves, so larger
+// sets launch plainly; griddep_sync() then returns at once.  Whole solves, plain
+// -> early: Jacobi-PCG FP64 33x45x37 21.6 -> 20.6 ms, 64^3 71.0 -> 69.4, 96^3 312
+// -> 309, 112^3 even; multigrid in FP32 48^3 6.23 -> 6.02, 64^3 8.69 -> 8.40, 96^3
+// 22.0 -> 21.7, 112^3 even; multigrid in FP64, whose stencils are twice the waves,
+// 32^3 3.43 -> 3.34, 56^3 13.3 -> 13.1, 64^3 12.0 -> 12.1, 80^3 24.4 -> 25.0, 96^3
+// 29.4 -> 30.7, 128^3 72.1 -> 73.6.
+constexpr long long kEarlyLaunchVoxels = 1 << 20, kEarlyLaunchVoxelsF64 = 200000;
+inline bool early_launch(const femh_config& c, long long nvox) {
+  const bool mg64 = c.solver == FEMH_GMG_PCG && c.precision == FEMH_FP64;
+  return nvox <= (mg64 ? kEarlyLaunchVoxelsF64 : kEarlyLaunchVoxels);
+}
 template <typename... P, typename... A>
 void launch(femh_handle* H, void (*fn)(P...), dim3 grid, unsigned block, size_t smem, A&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -287,7 +294,7 @@ void launch(femh_handle* H, void (*fn)(P...), dim3 grid, unsigned block, size_t 
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = H->nvox <= kEarlyLaunchVoxels ? 1 : 0;
+  cfg.numAttrs = early_launch(H->cfg, H->nvox) ? 1 : 0;
   CK(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
   LAUNCH_CHECK(H);
 }
