@@ -8,6 +8,8 @@
 // case), a unit being a contiguous node range of one cell, so that thousands
 // of cells of different sizes run in the same launch.
 #pragma once
+#include <type_traits>
+
 #include "femh_common.cuh"
 #include "stencil.cuh"
 
@@ -351,37 +353,45 @@ __global__ void k_cg_dir(const CellDesc* cells, const NodeUnit* units, TP* __res
   const CGState S = stt[cd.id * kNumRhs + rhs];
   if (!S.active) return;
   const double be = S.beta;
-  const bool mg = zvec && !S.fallback;
   constexpr int U = 4;   // as in k_cg_update
   const long long base = (long long)rhs * 3 * ntot + cd.off;
   const unsigned end = (unsigned)u.end, bd = blockDim.x;
+  // one loop per source of z: a choice at each load would part the loads
+  auto pass = [&](auto from_z) {
+    constexpr bool MG = decltype(from_z)::value;
 #pragma unroll 1
-  for (unsigned n0 = (unsigned)u.begin + threadIdx.x; n0 < end; n0 += U * bd) {
-    double zs[U][3];
-    LdT<TP> ps[U][3];
+    for (unsigned n0 = (unsigned)u.begin + threadIdx.x; n0 < end; n0 += U * bd) {
+      LdT<typename std::conditional<MG, TZ, TR>::type> zs[U][3];
+      LdT<TP> ps[U][3];
+      float ids[U];
 #pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const unsigned n = n0 + k * bd;
-      if (n >= end) break;
+      for (int k = 0; k < U; ++k) {
+        const unsigned n = n0 + k * bd;
+        if (n >= end) break;
+        if (!MG) ids[k] = invd[cd.off + n];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const long long o = base + c * ntot;
-        zs[k][c] = mg ? (double)ld_val(zvec + o + n) : (double)invd[cd.off + n] * (double)ld_val(r + o + n);
-        ps[k][c] = ld_val(p + o + n);
+        for (int c = 0; c < 3; ++c) {
+          const long long o = base + c * ntot;
+          if constexpr (MG) zs[k][c] = ld_val(zvec + o + n);
+          else zs[k][c] = ld_val(r + o + n);
+          ps[k][c] = ld_val(p + o + n);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        unsigned n = n0 + k * bd;
+        if (n >= end) break;
+        asm volatile("" : "+r"(n));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double z = MG ? (double)zs[k][c] : (double)ids[k] * (double)zs[k][c];
+          st_val(p + base + c * ntot + n, be == 0.0 ? z : z + be * (double)ps[k][c]);
+        }
       }
     }
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      unsigned n = n0 + k * bd;
-      if (n >= end) break;
-      asm volatile("" : "+r"(n));
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const double z = zs[k][c];
-        st_val(p + base + c * ntot + n, be == 0.0 ? z : z + be * (double)ps[k][c]);
-      }
-    }
-  }
+  };
+  if (zvec && !S.fallback) pass(std::true_type{});
+  else pass(std::false_type{});
 }
 
 // Sum of the partials of one (cell, rhs) over the cell's slot range: one warp,
