@@ -1083,19 +1083,19 @@ void prepare_operator(femh_handle* H) {
   {
     Prof prof_(H, "k_rhs", 0.0);
     k_rhs<true><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, H->kc64, H->d_ec, nullptr, L0.ntot,
-                                                  H->d_part_e, nullptr);
+                                                  H->d_part_e, H->d_part_n, nullptr);
     LAUNCH_CHECK(H);
   }
   {
     Prof prof_(H, "k_rhs_mean", 0.0);
-    k_rhs_mean<<<fin_blocks(H->ncells), 128, 0, s>>>(L0.d_cells, L0.d_nu_sb, L0.d_nu_se, H->d_part_e, H->d_mean,
+    k_rhs_mean<<<fin_blocks(H->ncells), 128, 0, s>>>(L0.d_nu_sb, L0.d_nu_se, H->d_part_e, H->d_part_n, H->d_mean,
                                                      H->ncells);
     LAUNCH_CHECK(H);
   }
   {
     Prof prof_(H, "k_rhs", 0.0);
     k_rhs<false><<<NODE_GRID(L0.all), 256, 0, s>>>(L0.d_cells, L0.all.d_nu, H->kc64, H->d_ec, H->b64, L0.ntot,
-                                                   nullptr, H->d_mean);
+                                                   nullptr, nullptr, H->d_mean);
     LAUNCH_CHECK(H);
   }
 }

@@ -176,27 +176,34 @@ __global__ void k_invblock(const CellDesc* cells, const NodeUnit* units, const T
 // without its net force.  The exact load has none, and the solver leaves the
 // three translations free, so it needs a load without one; and where the exact
 // load is zero (a uniform neighbourhood), rounding must not make one up: a
-// node's sum below its rounding bound, 8 u sum |kc_e g1|, is 0.  Two passes over the densities (8 B per node
-// each, against 144 B of load): SUM adds the load up, [slot][6][3] partials;
-// the other writes it less its mean per (cell, load case, component).
+// node's sum below its rounding bound, 8 u sum |kc_e g1|, is 0.  The net force
+// that rounding leaves is taken from the nodes in proportion to the stiffness
+// of their voxels, sum kc_e: in equal parts it would load soft voxels out of all
+// proportion to theirs (layers of 1 and 1e-12: C_11 off by 2e-9 of itself, now
+// below 1e-12) and voxels that have none.
+// Two passes over the densities (8 B per node each, against 144 B of load): SUM
+// adds the load up, [slot][6][3] partials, and the weights, [slot][6][2] (first
+// entry of load case 0); the other writes it less `mean`, its net force over
+// the sum of the weights per (cell, load case, component), times the weight.
 // One CTA per (unit, load case).
 template <bool SUM>
 __global__ void k_rhs(const CellDesc* cells, const NodeUnit* units, const double* kc64, const ElemConst* ec,
                       double* __restrict__ b, long long ntot, double* __restrict__ part,
-                      const double* __restrict__ mean) {
+                      double* __restrict__ wpart, const double* __restrict__ mean) {
   const NodeUnit u = units[blockIdx.x];
   const int I = blockIdx.y;
   const CellDesc cd = cells[u.cell];
-  double v[3] = {0.0, 0.0, 0.0};
+  double v[4] = {0.0, 0.0, 0.0, 0.0};   // net force, sum of the weights
   #pragma unroll 4
   for (long long n = u.begin + threadIdx.x; n < u.end; n += blockDim.x) {
     int i, j, k;
     node_ijk(n, cd.ny, cd.nz, i, j, k);
-    double acc[3] = {0, 0, 0}, size[3] = {0, 0, 0};
+    double acc[3] = {0, 0, 0}, size[3] = {0, 0, 0}, w = 0.0;
 #pragma unroll
     for (int a = 0; a < 8; ++a) {
       const double ke = kc64[cd.off + lin(wrap(i - ((a >> 2) & 1), cd.nx), wrap(j - ((a >> 1) & 1), cd.ny),
                                           wrap(k - (a & 1), cd.nz), cd.ny, cd.nz)];
+      w += ke;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         acc[c] += ke * ec->g1[I][3 * a + c];
@@ -207,15 +214,18 @@ __global__ void k_rhs(const CellDesc* cells, const NodeUnit* units, const double
     for (int c = 0; c < 3; ++c) {
       const double f = fabs(acc[c]) <= 8.0 * 1.1102230246251565e-16 * size[c] ? 0.0 : -cd.h * acc[c];
       if (SUM) v[c] += f;
-      else b[((long long)I * 3 + c) * ntot + cd.off + n] = f - mean[(cd.id * kNumRhs + I) * 3 + c];
+      else b[((long long)I * 3 + c) * ntot + cd.off + n] = f - mean[(cd.id * kNumRhs + I) * 3 + c] * w;
     }
+    if (SUM) v[3] += w;
   }
   if (SUM) {
-    __shared__ double red[32 * 3];
-    block_reduce<3>(v, red);
-    if (threadIdx.x == 0)
+    __shared__ double red[32 * 4];
+    block_reduce<4>(v, red);
+    if (threadIdx.x == 0) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) part[((long long)u.slot * kNumRhs + I) * 3 + c] = v[c];
+      if (I == 0) wpart[(long long)u.slot * kNumRhs * 2] = v[3];
+    }
   }
 }
 
@@ -281,8 +291,8 @@ k_cg_update(const CellDesc* cells, const NodeUnit* units, TV* __restrict__ x, TV
     // A thread issues the loads of U nodes before its first store, which later
     // loads cannot pass.  The stores' addresses are formed anew: kept from the
     // loads they would take as many registers as the values.  FP64 with U = 4
-    // spills at the 128 registers that two CTAs leave (33 x 45 x 37, a whole
-    // Jacobi iteration: U = 1 39.9, 2 39.6, 4 41.8 us).
+    // spills at the 128 registers that two CTAs leave (Jacobi solves, U = 1, 2, 4:
+    // 32^3 7.74, 7.53, 7.90 ms; 33x45x37 18.97, 18.97, 20.03).
     constexpr int U = sizeof(TV) == 8 ? 2 : 4;
     const long long base = (long long)rhs * 3 * ntot + cd.off;
     const unsigned end = (unsigned)u.end, bd = blockDim.x;
@@ -1734,15 +1744,16 @@ __global__ void k_param_sum(const int* __restrict__ ptr, const int* __restrict__
 }
 
 
-// Mean load per (cell, load case, component) from k_rhs's sums.
-__global__ void k_rhs_mean(const CellDesc* cells, const int* slot_begin, const int* slot_end, const double* part,
+// Net force over the sum of the weights per (cell, load case, component), from
+// k_rhs's sums.
+__global__ void k_rhs_mean(const int* slot_begin, const int* slot_end, const double* part, const double* wpart,
                            double* mean, int ncells) {
   FIN_PROLOGUE
-  const double nn = (double)cells[cell].nx * cells[cell].ny * cells[cell].nz;
+  const double w = sum_slots(wpart, slot_begin[cell], slot_end[cell], 0, 2, 0);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const double v = sum_slots(part, slot_begin[cell], slot_end[cell], rhs, 3, c);
-    if (lead) mean[t * 3 + c] = v / nn;
+    if (lead) mean[t * 3 + c] = w > 0.0 ? v / w : 0.0;
   }
 }
 

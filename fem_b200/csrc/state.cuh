@@ -203,7 +203,7 @@ struct femh_handle {
   unsigned long long fmap_key = 0;
   int fmap_nparam = -1;
   double* d_nrm = nullptr;      // [ncells][6]
-  double* d_mean = nullptr;     // [ncells][6][3] mean load (k_rhs)
+  double* d_mean = nullptr;     // [ncells][6][3] net force of the load over its weights (k_rhs)
   bool solved = false;
   bool have_x = false;   // x64 holds the last solution of these cells (warm starts)
   std::vector<double> C_last;

@@ -41,3 +41,17 @@ def test_dense_solve_takes_a_step_or_two(name, e_min, kw):
     assert info["status"] == 0
     assert max(info["iterations"]) <= 3
     assert np.abs(C - Cj).max() <= 1e-8 * np.abs(Cj).max()
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(precision=femh.MIXED_PC), dict(block_cg=0)])
+def test_load_of_soft_layers(kw):
+    """Layers of 1 and 1e-12 in series: C_11 in closed form.  It is the soft
+    layers' alone, so a net force of rounding size (1e-17) left on their nodes
+    shows at 2e-9 of it; the direct solve and the energy sum round at 1e-13."""
+    e = 1e-12
+    rho = np.zeros((5, 7, 9))
+    rho[:2] = 1
+    C, info = femh.Engine(E_min=e, autotune=0, **kw).homogenize(rho)
+    m = 0.7 / (1.3 * 0.4)   # (1 - nu) / ((1 + nu) (1 - 2 nu)), nu = 0.3
+    exact = 1.0 / (0.4 / m + 0.6 / (e * m))
+    assert info["status"] == 0 and abs(C[0, 0] / exact - 1) <= 1e-10
